@@ -432,7 +432,11 @@ int run_band_multi(const saru_batch *calls, const saru_result *res, int ncalls, 
   }
   a.counter = reinterpret_cast<int *>(scratch);
   a.planes = reinterpret_cast<uint8_t *>(scratch) + saru::kCounterBytes;
-  SARU_CUDA(saru::launch_band_kernel(a, s));
+  if (saru::diag_launch(max_m)) {
+    SARU_CUDA(saru::launch_diag_kernel(a, sm_count(dev), smem_per_sm(dev), tn.ctas_per_sm, s));
+  } else {
+    SARU_CUDA(saru::launch_band_kernel(a, s));
+  }
   g_launches.fetch_add(1);
   g_thread_launches += 1;
   return SARU_OK;

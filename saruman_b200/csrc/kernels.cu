@@ -1,12 +1,15 @@
 // kernels.cu -- sm_100a kernels of the alignment stage.
 //
-//  saru_band_kernel           the production path: persistent warps over
-//                             32-candidate tiles (one lane per candidate),
-//                             bit-parallel banded fill (saru_core.cuh) with
-//                             2-bit traceback decisions, traceback and slot
-//                             strings or compact records on the device; a
-//                             launch covers segments (calls, or slices
-//                             [t0, t1) of one call) of 32- or 64-bit bands.
+//  saru_diag_kernel           the production path for reads up to 255 bases:
+//                             persistent warps over 32-candidate tiles (one
+//                             lane per candidate), furthest columns by
+//                             diagonal and error count (diag_tile.cuh),
+//                             traceback and slot strings or compact records
+//                             on the device; a launch covers segments (calls,
+//                             or slices [t0, t1) of one call).
+//  saru_band_kernel           the same for longer reads: bit-parallel banded
+//                             fill (saru_core.cuh) of 32- or 64-bit bands with
+//                             2-bit traceback decisions (band_tile.cuh).
 //  saru_full_fill_kernel      the exact full-rectangle path for inputs the
 //  saru_full_trace_kernel     banded kernel does not cover (other costs,
 //                             m <= 3k, k > 15, irregular windows): the
@@ -20,6 +23,7 @@
 
 #include "kernels.cuh"
 #include "band_tile.cuh"
+#include "diag_tile.cuh"
 #include "saru_core.cuh"
 
 namespace saru {
@@ -152,6 +156,305 @@ __global__ void __launch_bounds__(128, 4) saru_band_kernel(const __grid_constant
     if (status && lane == 0)
       atomicOr(g.status, (status & 1 ? kStatusIrregular : 0) | (status & 2 ? kStatusAlphabet : 0) |
                              (status & 4 ? kStatusOverflow : 0));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// diagonal kernel: persistent warps over warp tiles (diag_tile.cuh)
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ Quad load_quad(const uint8_t *p) {
+  const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+  return Quad{v.x, v.y, v.z, v.w};
+}
+
+// A tile of the launch with its lanes' offsets, loaded while the tile before
+// it is aligned.
+struct TileAhead {
+  int tile, seg;
+  int g1, r1, dir;    // the lane's offsets (inclusive) and flag
+  int gp, rp;         // lane 0: the offsets before the tile
+  int g_lim, r_lim;   // the last offsets of the segment
+};
+
+__device__ __forceinline__ long tile_first(const Segment &g, int tile) {
+  return g.t0 + 32L * (tile - g.tile_begin);
+}
+
+// Starts the loads of a tile (tile < total).
+__device__ __forceinline__ void tile_ahead(const KernelArgs &a, int tile, int lane,
+                                           TileAhead &x) {
+  x.tile = tile;
+  int lo = 0, hi = a.nseg - 1;  // last segment with tile_begin <= tile
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (a.segs[mid].tile_begin <= tile) lo = mid;
+    else hi = mid - 1;
+  }
+  x.seg = lo;
+  const Segment &g = a.segs[lo];
+  const long t0 = tile_first(g, tile);
+  const long t = t0 + lane < g.n ? t0 + lane : g.n - 1;
+  x.g1 = g.goff[t];
+  x.r1 = g.roff[t];
+  x.dir = g.dirs[t];
+  x.gp = x.rp = 0;
+  if (lane == 0 && t0 > 0) {
+    x.gp = g.goff[t0 - 1];
+    x.rp = g.roff[t0 - 1];
+  }
+  x.g_lim = g.goff[g.n - 1];
+  x.r_lim = g.roff[g.n - 1];
+}
+
+// The byte ranges of a tile whose offsets have arrived.
+__device__ __forceinline__ bool tile_span(const KernelArgs &a, const TileAhead &x, int count,
+                                          DiagSpan &s) {
+  const Segment &g = a.segs[x.seg];
+  s.g_lo = __shfl_sync(0xffffffffu, x.gp, 0);
+  s.r_lo = __shfl_sync(0xffffffffu, x.rp, 0);
+  s.g_hi = __shfl_sync(0xffffffffu, x.g1, 31);
+  s.r_hi = __shfl_sync(0xffffffffu, x.r1, 31);
+  s.g_lim = x.g_lim;
+  s.r_lim = x.r_lim;
+  return s.set(g.reads, g.genome, count, g.max_m, g.k);
+}
+
+// The whole 16-byte blocks of bytes [lo, hi) of an array to L2.
+__device__ __forceinline__ void prefetch_l2(const uint8_t *p, int lo, int hi) {
+  const uintptr_t b = ((uintptr_t)(p + lo) + 15) & ~(uintptr_t)15;
+  const uintptr_t e = (uintptr_t)(p + hi) & ~(uintptr_t)15;
+  if (b < e)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((uint32_t)(e - b))
+                 : "memory");
+}
+
+// Starts the copies of a tile's reads and windows to shared memory.
+__device__ __forceinline__ void stage_tile(const Segment &g, const DiagSpan &s, Sm reads,
+                                           Sm windows, int lane) {
+  auto copy16 = [](Sm d, const uint8_t *p) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d.a),
+                 "l"(__cvta_generic_to_global(p))
+                 : "memory");
+  };
+  stage_bytes(reads, g.reads, s.r_base, s.r_hi, s.r_lim, lane, copy16, load_quad);
+  stage_bytes(windows, g.genome, s.g_base, s.g_hi, s.g_lim, lane, copy16, load_quad);
+}
+
+// Levels and walk of a lane on its mismatch look-up P.
+template <typename RW, class X>
+__device__ __forceinline__ int diag_lane(const X &P, const DiagTable &T, RW eq, int reach,
+                                         DiagLane &l, WalkEnd &end, const GapMask &U,
+                                         const GapMask &Lf) {
+  const DiagExit x = lane_levels<RW>(l.c, P, T, eq, reach);
+  l.score = x.score;
+  if (x.score > T.k) return 0;
+  end = lane_diag_walk<RW>(l.c, P, T, x, eq, reach, U, Lf);
+  if (!end.bad) return 0;
+  end.n = 0;
+  return 4;
+}
+
+// From the tile's bit streams (in the table's place) to the lanes' walks.
+template <bool ROWS, bool ODD>
+__device__ __forceinline__ int diag_align(const uint8_t *reads, const uint8_t *genome, int k,
+                                          const DiagSpan &s, const DiagLayout &D, int lane,
+                                          Sm slice, DiagLane &l, WalkEnd &end, const GapMask &U,
+                                          const GapMask &Lf) {
+  using RW = typename DiagWord<ROWS>::type;
+  int st = 0;
+  const Sm table = slice + D.compare_bytes, sr = table, sw = sr + 12 * D.rw;
+  if (ODD) {
+    stream_odd(slice + D.raw, (int)(s.r_hi - s.r_base), sr + 8 * D.rw, lane);
+    stream_odd(slice + (D.raw + D.src_r), (int)(s.g_hi - s.g_base), sw + 8 * D.ww, lane);
+    __syncwarp();
+  }
+  const StreamWords R{sr, sr + 4 * D.rw, sr + 8 * D.rw, l.ok ? 32 + (int)(l.rs - s.r_base) : 32};
+  const StreamWords W{sw, sw + 4 * D.ww, sw + 8 * D.ww, l.ok ? 32 + (int)(l.gs - s.g_base) : 32};
+  const uint8_t *read = reads + l.rs, *win = genome + l.gs;
+  Extras x;
+  x.n = 0;
+  if (ODD && l.ok && !read_extras(R, D.nr, l.c.m, read, x)) {
+    st = 2;  // alphabet
+    l.ok = false;
+  }
+  const int m = l.ok ? l.c.m : 0, L = l.ok ? l.c.L : 0;
+  const MismatchRows M(slice, D, lane, k);
+  const Planes<ODD> P(slice, D, lane, k);
+  RW eq = 0;
+  if (ROWS) {
+    if (l.ok) eq = lane_rows<ODD>(R, W, l.c, read, win, x, D, M);
+  } else {
+    lane_planes<ODD>(R, D.nr, m, read, x, false, P.rd);
+    lane_planes<ODD>(W, D.nw, L, win, x, true, P.wn);
+  }
+  __syncwarp();
+  {  // table and gap masks (adjacent) start from zero
+    const int end16 = D.table_bytes + D.masks_bytes;
+    for (int i = 16 * lane; i < end16; i += 512) sm_st128(table + i, Quad{0, 0, 0, 0});
+  }
+  __syncwarp();
+  end = WalkEnd{0, 0, 0, false};
+  const DiagTable T(table, D, lane, k);
+  if (l.ok) {
+    if (ROWS) st |= diag_lane<RW>(M, T, eq, D.reach, l, end, U, Lf);
+    else st |= diag_lane<RW>(P, T, (RW)P.matches(m, D.reach), D.reach, l, end, U, Lf);
+  }
+  return st;
+}
+
+// One warp tile; `next`: the tile after it (its offsets arrive while this
+// one is aligned, its bytes go to L2 while this one's strings are written).
+template <bool ROWS>
+__device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &now, int next,
+                                         TileAhead &ahead, int lane, uint8_t *slice_p, Sm gaps) {
+  const Segment &g = a.segs[now.seg];
+  const int k = g.k;
+  const long t0 = tile_first(g, now.tile);
+  const int count = g.n - t0 < 32 ? (int)(g.n - t0) : 32;
+  int g0 = __shfl_up_sync(0xffffffffu, now.g1, 1), r0 = __shfl_up_sync(0xffffffffu, now.r1, 1);
+  if (lane == 0) {
+    g0 = now.gp;
+    r0 = now.rp;
+  }
+  DiagSpan s;
+  const bool fits = tile_span(a, now, 32, s);
+  DiagLane l;
+  int st = lane_candidate(s, g0, now.g1, r0, now.r1, now.dir, k, g.max_m,
+                          g.first_of_call && t0 + lane == 0, lane < count, l)
+               ? 0
+               : 1;
+  const DiagLayout D = diag_layout(g.max_m, k, ROWS);
+  const Sm slice = sm_at(slice_p);
+  uint32_t odd = 0;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+  if (fits) {
+    const Sm sr = slice + D.compare_bytes, sw = sr + 12 * D.rw;
+    odd = stream_planes(slice + D.raw, (int)(s.r_hi - s.r_base), sr, sr + 4 * D.rw, lane);
+    odd |= stream_planes(slice + (D.raw + D.src_r), (int)(s.g_hi - s.g_base), sw, sw + 4 * D.ww,
+                         lane);
+  }
+  const bool more = next < a.total_tiles;
+  if (more) tile_ahead(a, next, lane, ahead);
+  else ahead.tile = next;
+  // the next tile's bytes: to L2 while this one's strings are written, then
+  // to shared memory
+  DiagSpan sn;
+  bool fits_next = false;
+  auto prefetch = [&]() {
+    if (!more) return;
+    fits_next = tile_span(a, ahead, 32, sn);
+    if (fits_next && lane == 0) {
+      const Segment &h = a.segs[ahead.seg];
+      prefetch_l2(h.genome, sn.g_lo, sn.g_hi);
+      prefetch_l2(h.reads, sn.r_lo, sn.r_hi);
+    }
+  };
+  auto finish = [&]() {
+    if (!more || !fits_next) return;
+    const Segment &h = a.segs[ahead.seg];
+    const DiagLayout N = diag_layout(h.max_m, h.k, ROWS);
+    stage_tile(h, sn, slice + N.raw, slice + (N.raw + N.src_r), lane);
+  };
+  if (!fits) {  // offsets no regular call can have: report, do not stage
+    if (lane < count) g.scores[t0 + lane] = k + 1;
+    prefetch();
+    finish();
+    return 1;
+  }
+  const Sm masks = slice + (D.compare_bytes + D.table_bytes + 4 * lane);
+  const GapMask U{masks}, Lf{masks + D.mwords * 128};
+  __syncwarp();
+  WalkEnd end;
+  if (__any_sync(0xffffffffu, odd != 0))
+    st |= diag_align<ROWS, true>(g.reads, g.genome, k, s, D, lane, slice, l, end, U, Lf);
+  else
+    st |= diag_align<ROWS, false>(g.reads, g.genome, k, s, D, lane, slice, l, end, U, Lf);
+  __syncwarp();
+  prefetch();
+  if (lane < count) g.scores[t0 + lane] = l.score;
+  if (g.records) {  // compact records straight to global memory
+    if (lane < count) {
+      uint32_t *rec = reinterpret_cast<uint32_t *>(g.records + (t0 + lane) * g.rec_bytes);
+      const int nwords = (int)(g.rec_bytes >> 2);
+      rec[0] = (uint32_t)end.n | (end.bad ? 0x10000u : 0u);
+      record_words(end.n, nwords, U, Lf, [&](int w, uint32_t v) { rec[w] = v; });
+    }
+    finish();
+    return st;
+  }
+  // the strings: both sources staged again, then one array after the other
+  // written over zeros and its slot range copied out
+  const Sm out = slice + (D.src_r + D.src_w);
+  auto st16 = [](uint8_t *d, const uint8_t *p) {
+    *reinterpret_cast<uint4 *>(d) = *reinterpret_cast<const uint4 *>(p);
+  };
+  const long s_lo = s.g_lo + k * t0, s_hi = s.g_hi + k * (t0 + count);
+  const int slot = l.gs - s.g_lo + k * lane;  // the lane's slot from s_lo
+  stage_tile(g, s, slice + 16, slice + (D.src_r + 16), lane);
+  for (int pass = 0; pass < 2; ++pass) {
+    uint8_t *to = pass ? g.genome_aln : g.read_aln;
+    const long o_base = stage_base(to, s_lo);
+    for (int i = 16 * lane; i < D.out_bytes; i += 512) sm_st128(out + i, Quad{0, 0, 0, 0});
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    if (end.n) {
+      const int from = pass ? D.src_r + 16 + (int)(l.gs - s.g_base) + end.row
+                            : 16 + (int)(l.rs - s.r_base) + end.col;
+      expand_masked(out + (slot + (int)(s_lo - o_base)), end.n, slice + from, pass ? Lf : U, gaps);
+    }
+    __syncwarp();
+    stage_out(to, slice_p + (D.src_r + D.src_w), s_lo, s_hi, o_base, lane, st16);
+    __syncwarp();
+  }
+  finish();
+  return st;
+}
+
+// 16 warps an SM: 104 registers a thread leave room for more, but the slices
+// do not (14.2 KB at 100 bp, k = 5).  Held to 3 or 5 CTAs of 4 warps: 332 or
+// 294 us against 291 for 930k candidates of 100 bp.
+constexpr int kDiagCtas = 4;
+constexpr int kDiagWarpsPerSm = 4 * kDiagCtas;
+
+// Persistent warps: the first tile of a warp is its own number, later ones
+// come from the launch's counter (none: the grid has a warp for every tile).
+template <bool ROWS>
+__global__ void __launch_bounds__(128, kDiagCtas)
+    saru_diag_kernel(const __grid_constant__ KernelArgs a) {
+  extern __shared__ uint4 smem_v[];
+  __shared__ uint32_t gaps[16];
+  if (threadIdx.x < 16) gaps[threadIdx.x] = gap_select((int)threadIdx.x);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int warps = blockDim.x >> 5;
+  uint8_t *slice = reinterpret_cast<uint8_t *>(smem_v) + (long)(threadIdx.x >> 5) * a.warp_smem;
+  const int first = (int)(blockIdx.x * warps + (threadIdx.x >> 5));
+  if (first >= a.total_tiles) return;
+  TileAhead now;
+  tile_ahead(a, first, lane, now);
+  {
+    const Segment &g = a.segs[now.seg];
+    const DiagLayout D = diag_layout(g.max_m, g.k, ROWS);
+    DiagSpan s;
+    const Sm raw = sm_at(slice) + D.raw;
+    if (tile_span(a, now, 32, s)) stage_tile(g, s, raw, raw + D.src_r, lane);
+  }
+  while (now.tile < a.total_tiles) {
+    int next = (int)a.total_tiles;
+    if (a.counter) {
+      if (lane == 0) next = (int)gridDim.x * warps + atomicAdd(a.counter, 1);
+      next = __shfl_sync(0xffffffffu, next, 0);
+    }
+    TileAhead ahead;
+    int status = diag_tile<ROWS>(a, now, next, ahead, lane, slice, sm_at(gaps));
+    status = __reduce_or_sync(0xffffffffu, status);
+    if (status && lane == 0)
+      atomicOr(a.segs[now.seg].status,
+               (status & 1 ? kStatusIrregular : 0) | (status & 2 ? kStatusAlphabet : 0) |
+                   (status & 4 ? kStatusOverflow : 0));
+    now = ahead;
   }
 }
 
@@ -297,12 +600,90 @@ cudaError_t allow_smem() {
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lk(g_attr_mu);
   if ((g_attr_done >> dev) & 1u) return cudaSuccess;
-  e = cudaFuncSetAttribute(saru_band_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kMaxCtaSmem);
+  const int attr = cudaFuncAttributeMaxDynamicSharedMemorySize, most = (int)kMaxCtaSmem;
+  e = cudaFuncSetAttribute(saru_band_kernel, (cudaFuncAttribute)attr, most);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(saru_diag_kernel<true>, (cudaFuncAttribute)attr, most - 64);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(saru_diag_kernel<false>, (cudaFuncAttribute)attr, most - 64);
   if (e == cudaSuccess) g_attr_done |= 1ull << dev;
   return e;
 }
 }  // namespace
+
+// The diagonal kernel takes every launch whose reads fit its byte columns;
+// the banded one the longer reads.
+bool diag_launch(int max_m) { return max_m <= kDiagMaxM; }
+
+// The largest slice a launch's segments need (a slice does not grow with
+// the read length and k in every case, so it is not the longest read's).
+long diag_slice(const KernelArgs &a, bool rows) {
+  long most = 0;
+  for (int i = 0; i < a.nseg; ++i) {
+    const long s = diag_layout(a.segs[i].max_m, a.segs[i].k, rows).slice;
+    if (s > most) most = s;
+  }
+  return most;
+}
+
+// Whether a launch looks its mismatches up in rows: one word has a bit per
+// diagonal -k .. 5k/2 up to k = 9, a row's columns past m must fit a byte, and
+// the slice must leave room for enough warps.  Rows take 68 us where planes
+// take 88 for 176k candidates of 100 bp at k = 5 (14 KB a slice against 16),
+// 70 against 50 for 41k of 133 bp at k = 8 (29 KB against 21).
+constexpr long kRowsSlice = 20 * 1024;
+bool diag_rows(const KernelArgs &a) {
+  return a.max_k <= 9 && a.max_m <= 200 && diag_slice(a, true) <= kRowsSlice;
+}
+
+// CTAs of w warps (shared memory w slices) an SM holds.
+int diag_ctas_per_sm(int w, long slice, int smem_per_sm) {
+  const long by_smem = smem_per_sm / (w * slice + 64 + 1024);
+  const long by_regs = kDiagWarpsPerSm / w;
+  return (int)(by_smem < by_regs ? by_smem : by_regs);
+}
+
+// Warps per CTA: what was asked for, else the count that keeps the most
+// warps on an SM (large slices: CTAs of one warp pack best).
+int diag_warps(long slice, int warps_req, int smem_per_sm) {
+  const int most = (int)((kMaxCtaSmem - 64) / slice);
+  if (warps_req >= 1) return warps_req < most ? warps_req : most;
+  int best = 0, warps = 1;
+  for (int w = most < 4 ? most : 4; w >= 1; --w) {
+    const int n = w * diag_ctas_per_sm(w, slice, smem_per_sm);
+    if (n > best) {
+      best = n;
+      warps = w;
+    }
+  }
+  return warps;
+}
+
+cudaError_t launch_diag_kernel(KernelArgs &a, int sms, int smem_per_sm, int ctas_cap,
+                               cudaStream_t s) {
+  if (a.nseg < 1 || a.nseg > kMaxSegs) return cudaErrorInvalidValue;
+  cudaError_t e = allow_smem();
+  if (e != cudaSuccess) return e;
+  const bool rows = diag_rows(a);
+  a.warp_smem = diag_slice(a, rows);
+  const int warps = diag_warps(a.warp_smem, a.warps_req, smem_per_sm);
+  if (warps < 1) return cudaErrorInvalidValue;
+  long per_sm = diag_ctas_per_sm(warps, a.warp_smem, smem_per_sm);
+  if (per_sm < 1) per_sm = 1;
+  if (ctas_cap >= 1 && per_sm > ctas_cap) per_sm = ctas_cap;
+  const long ctas = (a.total_tiles + warps - 1) / warps;
+  a.grid = ctas < sms * per_sm ? ctas : sms * per_sm;
+  if (a.total_tiles <= a.grid * warps) {
+    a.counter = nullptr;  // a warp for every tile
+  } else {
+    e = cudaMemsetAsync(a.counter, 0, sizeof(int), s);
+    if (e != cudaSuccess) return e;
+  }
+  const size_t smem = (size_t)(a.warp_smem * warps);
+  if (rows) saru_diag_kernel<true><<<(unsigned)a.grid, 32 * warps, smem, s>>>(a);
+  else saru_diag_kernel<false><<<(unsigned)a.grid, 32 * warps, smem, s>>>(a);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_band_kernel(KernelArgs &a, cudaStream_t s) {
   const BandLayout L = band_layout(a.max_m, a.max_k, a.warps_req, a.wide_any != 0);

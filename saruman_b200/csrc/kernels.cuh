@@ -111,6 +111,9 @@ long band_grid(int sms, long n, const BandLayout &L, int smem_per_sm, int ctas_c
 size_t band_scratch_bytes(long grid, int max_m, int k, bool wide,
                           int warps_req = 0);  // counter + planes
 cudaError_t launch_band_kernel(KernelArgs &a, cudaStream_t s);
+bool diag_launch(int max_m);  // whether a launch's reads go to the diagonal kernel
+cudaError_t launch_diag_kernel(KernelArgs &a, int sms, int smem_per_sm, int ctas_cap,
+                               cudaStream_t s);
 cudaError_t launch_full_kernels(const FullArgs &a, cudaStream_t s);
 
 }  // namespace saru

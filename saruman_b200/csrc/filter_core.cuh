@@ -244,4 +244,122 @@ SARU_HD void filter_read(const FilterShape &S, int dr, const Lists &L, Perfect p
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same filter, position by position
+// ---------------------------------------------------------------------------
+//
+// Only the pair that brings a position's count to the threshold is recorded,
+// and its flag and start depend on the two q-grams, not on the error zone.
+// So a position needs, per pair of q-grams, how many hits its zones have: one
+// search of a list for a range of values instead of one per zone.
+
+// A range of genome positions [lo, lo + width], in the lists' 32 bits.  (The
+// zones of a position near the genome's start that lie before it hold no
+// list value: 32-bit wraps of them are past every genome.)
+struct PosRange {
+  uint32_t lo, width;
+  bool none;
+  SARU_HD PosRange(int64_t from, int64_t to)
+      : lo((uint32_t)(from > 0 ? from : 0)), width((uint32_t)(to - (from > 0 ? from : 0))),
+        none(to < 0) {}
+  SARU_HD bool in(uint32_t v) const { return v - lo <= width && !none; }
+};
+
+// Elements of list x from index `from` on in range r, counted up to `most`
+// (list values ascend).  Lists: value(x, i), element i < len(x); lower(x,
+// from, v), the first index >= from whose value is >= v (len(x) for none).
+template <class Lists>
+SARU_HD int count_range(const Lists &L, int x, uint32_t from, const PosRange &r, int most) {
+  const uint32_t len = L.len(x);
+  int n = 0;
+  for (uint32_t i = L.lower(x, from, r.lo); i < len && n < most; ++i, ++n)
+    if (!r.in(L.value(x, i))) break;
+  return n;
+}
+
+// Hits of all error zones of a first-pass pair: list b scanned from index
+// `off` (scan_from_at) for the values of r.
+template <class Lists>
+SARU_HD int pair_hits(const Lists &L, int b, int nlists, uint32_t off, const PosRange &r,
+                      int most) {
+  const uint32_t len = L.len(b);
+  if (len >= 1 || off == 0 || b + 1 >= nlists) {
+    const uint32_t v0 = L.at(b, off);
+    if (v0 == 0) return 0;
+    int n = r.in(v0);
+    if (len >= 1) return n >= most ? n : n + count_range(L, b, 1, r, most - n);
+    for (uint32_t i = 1;; ++i) {  // an empty list: the walk runs into the next lists
+      const uint32_t v = L.at(b, i);
+      if (v == 0) return n;
+      n += r.in(v);
+    }
+  }
+  const uint32_t len1 = L.len(b + 1);
+  const uint32_t v0 =
+      off - 1 < len1 ? L.value(b + 1, off - 1) : (off - 1 == len1 ? 0u : L.at(b, off));
+  if (v0 == 0) return 0;
+  const int n = r.in(v0);
+  if (len1 == 0 || n >= most || L.value(b + 1, 0) == 0) return n;
+  return n + count_range(L, b + 1, 0, r, most - n);
+}
+
+// Whether position `off` (value pa) of first-half q-gram a reaches the
+// threshold, and the flag and start recorded for it.
+template <class Lists>
+SARU_HD bool position_hit(const FilterShape &S, int dr, const Lists &L, int a, uint32_t off,
+                          uint32_t pa, int &flag, int &start) {
+  const int k = S.k, half = S.half, q = S.q;
+  const int first = a == 0 ? 1 : 0;
+  const int gs = (int)(pa - ((uint32_t)a * q + 1));
+  int need = S.tresh - 1;  // hits up to the one that reaches the threshold
+  if (need < 1) return false;
+  for (int b = a + 1; b < half; ++b) {
+    const int64_t want = (int64_t)gs + (int64_t)b * q + 1;
+    need -= pair_hits(L, b, S.P, off, PosRange(want - k, want + k), need);
+    if (need > 0) continue;
+    if (first) {
+      flag = 1 + dr;
+      start = gs + 1;
+    } else {
+      flag = 3 + dr;
+      start = gs - k + 1;
+    }
+    return true;
+  }
+  for (int b = 0; b < half; ++b) {
+    int lim = half - 1 - b - a;
+    if (lim < 0) lim = -lim;
+    const uint32_t ns = (uint32_t)(half - b - 1) * q + 1 + S.rest;
+    if (L.len(half + b) == 0 || L.value(half + b, 0) == 0) continue;
+    const int64_t want = (int64_t)gs + (int64_t)ns;
+    need -= count_range(L, half + b, 0, PosRange(want - lim, want + lim), need);
+    if (need > 0) continue;
+    if (first) {
+      flag = 1 + dr;
+      start = gs + 1;
+    } else {
+      flag = (b == 0 ? ((int)(ns + q) > S.m ? 3 : 2) : 3) + dr;
+      start = gs - k + 1;
+    }
+    return true;
+  }
+  return false;
+}
+
+// What a kept position (pc, fc) decides about a new one: 0 nothing, 1
+// dropped, 2 its flag replaces the kept one's, 3 dropped as equal
+// (filter_record's tests in their order).
+//
+// The distances are taken modulo 2^32: pc - start is off by 2^32 only when
+// both positions are near 2^31 and of opposite signs, and then -pc - start is
+// in the same distance.
+SARU_HD int kept_decides(int pc, int fc, int k, int start, int flag) {
+  const uint32_t p = (uint32_t)pc, s = (uint32_t)start, w = 2u * (uint32_t)k;
+  const bool near_it = p - s + (uint32_t)k <= w || (uint32_t)k - p - s <= w;
+  if (near_it && fc <= flag) return 1;
+  if (!near_it || (fc > 3) != (flag > 3)) return 0;
+  if (pc == start) return 2;
+  return p + s == 0u ? 3 : 0;
+}
+
 }  // namespace saru

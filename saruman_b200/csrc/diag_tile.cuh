@@ -168,11 +168,11 @@ SARU_HD int low_bit(uint64_t x) {
 // ---------------------------------------------------------------------------
 //
 //   [compare: what a lane looks its mismatches up in, see below]
-//   [table: a row of `width` x 32 bytes per level | before: the bit streams]
+//   [table: 32 bytes per diagonal and level, see DiagTable]
 //   [gap masks: 2 x mwords x 32 words, and a word more]
-// The tile's bytes lie over the first two (not over the streams) until the
-// streams are made; after the walk they come back as the strings' sources,
-// with the output staging behind them.
+// The tile's bytes lie over the front of the first two and their bit streams
+// at the end of them until the compare part is made; after the walk the bytes
+// come back as the strings' sources, with the output staging behind them.
 //
 // Two forms of the compare part: `rows`, a lane's mismatch bits of every
 // diagonal (a look-up is two words and a shift), and planes, its read's and
@@ -183,16 +183,23 @@ struct DiagLayout {
   int nr, nw;       // words a lane holds of its read / window
   int reach;        // highest diagonal of any level (5k/2), see diag_hi
   int diags;        // rows of mismatches: -k .. reach, an even number of them
-  int width;        // diagonals of a table row: -k-1 .. reach + 2
   int rw, ww;       // words of one plane's bit stream over the tile's reads / windows
   int mwords;       // words of a gap mask
   int src_r, src_w; // room for the tile's reads and windows
-  int raw;          // where they lie until the streams are made
   int out_bytes;    // one output string array of the tile
+  int streams;      // where the bit streams lie
   int compare_bytes, table_bytes, masks_bytes, slice;
 };
 
 SARU_HD int up16(int x) { return (x + 15) & ~15; }
+
+// Cells before level e in the table: level i holds diagonals -i - 2 .. hi(i)
+// + 2 with hi(i) = min(2k + i, 3k - i) (diag_hi at so = eo = k; the next level
+// and the walk look at the two beyond on either side).
+SARU_HD int table_cells(int e, int k) {
+  const int h = k / 2 + 1, x = e < h ? e : h;
+  return x * (2 * k + 4 + x) + (e - x) * (3 * k + 5);
+}
 
 SARU_HD DiagLayout diag_layout(int max_m, int k, bool rows) {
   DiagLayout D;
@@ -200,7 +207,6 @@ SARU_HD DiagLayout diag_layout(int max_m, int k, bool rows) {
   D.diags = (k + D.reach + 2) & ~1;
   D.nr = ((max_m + 1) >> 5) + 1;
   D.nw = ((max_m + 2 + D.reach) >> 5) + 1;
-  D.width = k + D.reach + 4;
   D.rw = max_m + D.nr + 4;
   D.ww = max_m + 2 * k + D.nw + 4;
   D.mwords = ((31 + max_m + 3 * k) >> 5) + 1;
@@ -211,17 +217,16 @@ SARU_HD DiagLayout diag_layout(int max_m, int k, bool rows) {
   D.compare_bytes =
       rows ? (D.diags * D.nr + 2) * 128 : (D.nr + D.nw + 2) * 512;
   const int streams = up16(3 * 4 * (D.rw + D.ww));
-  D.table_bytes = (k > 0 ? k : 1) * D.width * 32;
-  if (D.table_bytes < streams) D.table_bytes = streams;
+  D.table_bytes = table_cells(k > 0 ? k : 1, k) * 32;
   D.masks_bytes = (2 * D.mwords + 1) * 128;
-  const int strings = D.src_r + D.src_w + D.out_bytes;
-  if (D.compare_bytes + D.table_bytes < strings) D.table_bytes = strings - D.compare_bytes;
-  D.raw = 0;
-  if (D.compare_bytes < D.src_r + D.src_w) {
-    D.raw = D.compare_bytes + streams;
-    if (D.table_bytes < streams + D.src_r + D.src_w) D.table_bytes = streams + D.src_r + D.src_w;
-  }
-  D.slice = D.compare_bytes + D.table_bytes + D.masks_bytes;
+  int front = D.compare_bytes + D.table_bytes;
+  const int raw = D.src_r + D.src_w;
+  if (front < raw + D.out_bytes) front = raw + D.out_bytes;
+  if (front < raw + streams) front = raw + streams;
+  if (front < D.compare_bytes + streams) front = D.compare_bytes + streams;
+  D.table_bytes = front - D.compare_bytes;
+  D.streams = front - streams;
+  D.slice = front + D.masks_bytes;
   return D;
 }
 
@@ -525,14 +530,16 @@ SARU_HD void lane_planes(const StreamWords &s, int entries, int len, const uint8
 // column of diagonal d with a value <= e, 0 if none is known; columns end at
 // m - 1 (the last one has rules of its own).
 struct DiagTable {
-  Sm zero;  // diagonal 0 of level 0
-  int row;  // bytes of a row
+  Sm base;  // diagonal 0 of level 0
   int k;
-  SARU_HD DiagTable(Sm table, const DiagLayout &D, int lane, int k_)
-      : zero(table + ((k_ + 1) * 32 + lane)), row(D.width * 32), k(k_) {}
-  SARU_HD Sm cell(int e, int d) const { return zero + (e * row + d * 32); }
+  SARU_HD DiagTable(Sm table, int lane, int k_) : base(table + (lane + 64)), k(k_) {}
+  SARU_HD Sm cell(int e, int d) const { return base + (table_cells(e, k) + e + d) * 32; }
   SARU_HD int at(int e, int d) const { return sm_ld8(cell(e, d)); }
-  SARU_HD bool has(int d) const { return (unsigned)((d + k + 1) * 32) < (unsigned)row; }
+  // whether level e has a cell for d
+  SARU_HD bool has(int e, int d) const {
+    const int hi = 2 * k + e < 3 * k - e ? 2 * k + e : 3 * k - e;
+    return d >= -e - 2 && d <= hi + 2;
+  }
 };
 
 // Diagonals of level e that can still reach the end within k errors: a path
@@ -768,7 +775,7 @@ SARU_HD WalkEnd lane_diag_walk(const Cand &c, const X &P, const DiagTable &T, co
   U.range(0, nup);
   int how = x.how;
   if (how == OP_UP) {  // below the free rows of the last column: every step up costs one
-    auto at_end = [&](int e, int dd) { return e >= 0 && T.has(dd) && T.at(e, dd) >= m; };
+    auto at_end = [&](int e, int dd) { return e >= 0 && T.has(e, dd) && T.at(e, dd) >= m; };
     auto diag = [&](int e, int dd) {
       return at_end(e - 1, dd) || (at_end(e, dd) && dd >= -k && ((eq >> (RW)(reach - dd)) & RW(1)));
     };
@@ -804,7 +811,7 @@ SARU_HD WalkEnd lane_diag_walk(const Cand &c, const X &P, const DiagTable &T, co
       col = lo;
       break;
     }
-    if (!T.has(d) || d + k < 0) {
+    if (!T.has(v - 1, d) || !T.has(v - 1, d - 1)) {
       bad = true;
       break;
     }

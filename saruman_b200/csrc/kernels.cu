@@ -241,6 +241,38 @@ __device__ __forceinline__ void stage_tile(const Segment &g, const DiagSpan &s, 
   stage_bytes(windows, g.genome, s.g_base, s.g_hi, s.g_lim, lane, copy16, load_quad);
 }
 
+// The lanes' compare parts from the tile's bit streams; the alphabet status
+// bit.  eq: row_matches (rows form).
+template <bool ROWS, bool ODD>
+__device__ __forceinline__ int diag_compare(const Segment &g, const DiagSpan &s,
+                                            const DiagLayout &D, int lane, Sm slice, DiagLane &l,
+                                            uint32_t &eq) {
+  int st = 0;
+  const Sm sr = slice + D.streams, sw = sr + 12 * D.rw;
+  if (ODD) {
+    stream_odd(slice, (int)(s.r_hi - s.r_base), sr + 8 * D.rw, lane);
+    stream_odd(slice + D.src_r, (int)(s.g_hi - s.g_base), sw + 8 * D.ww, lane);
+    __syncwarp();
+  }
+  const StreamWords R{sr, sr + 4 * D.rw, sr + 8 * D.rw, l.ok ? 32 + (int)(l.rs - s.r_base) : 32};
+  const StreamWords W{sw, sw + 4 * D.ww, sw + 8 * D.ww, l.ok ? 32 + (int)(l.gs - s.g_base) : 32};
+  const uint8_t *read = g.reads + l.rs, *win = g.genome + l.gs;
+  Extras x;
+  x.n = 0;
+  if (ODD && l.ok && !read_extras(R, D.nr, l.c.m, read, x)) {
+    st = 2;  // alphabet
+    l.ok = false;
+  }
+  if (ROWS) {
+    if (l.ok) eq = lane_rows<ODD>(R, W, l.c, read, win, x, D, MismatchRows(slice, D, lane, g.k));
+  } else {
+    const Planes<ODD> P(slice, D, lane, g.k);
+    lane_planes<ODD>(R, D.nr, l.ok ? l.c.m : 0, read, x, false, P.rd);
+    lane_planes<ODD>(W, D.nw, l.ok ? l.c.L : 0, win, x, true, P.wn);
+  }
+  return st;
+}
+
 // Levels and walk of a lane on its mismatch look-up P.
 template <typename RW, class X>
 __device__ __forceinline__ int diag_lane(const X &P, const DiagTable &T, RW eq, int reach,
@@ -255,52 +287,33 @@ __device__ __forceinline__ int diag_lane(const X &P, const DiagTable &T, RW eq, 
   return 4;
 }
 
-// From the tile's bit streams (in the table's place) to the lanes' walks.
-template <bool ROWS, bool ODD>
-__device__ __forceinline__ int diag_align(const uint8_t *reads, const uint8_t *genome, int k,
-                                          const DiagSpan &s, const DiagLayout &D, int lane,
-                                          Sm slice, DiagLane &l, WalkEnd &end, const GapMask &U,
-                                          const GapMask &Lf) {
+// From the tile's bit streams to the lanes' walks.
+template <bool ROWS>
+__device__ __forceinline__ int diag_align(const Segment &g, const DiagSpan &s, const DiagLayout &D,
+                                          bool odd, int lane, Sm slice, DiagLane &l, WalkEnd &end,
+                                          const GapMask &U, const GapMask &Lf) {
   using RW = typename DiagWord<ROWS>::type;
-  int st = 0;
-  const Sm table = slice + D.compare_bytes, sr = table, sw = sr + 12 * D.rw;
-  if (ODD) {
-    stream_odd(slice + D.raw, (int)(s.r_hi - s.r_base), sr + 8 * D.rw, lane);
-    stream_odd(slice + (D.raw + D.src_r), (int)(s.g_hi - s.g_base), sw + 8 * D.ww, lane);
-    __syncwarp();
-  }
-  const StreamWords R{sr, sr + 4 * D.rw, sr + 8 * D.rw, l.ok ? 32 + (int)(l.rs - s.r_base) : 32};
-  const StreamWords W{sw, sw + 4 * D.ww, sw + 8 * D.ww, l.ok ? 32 + (int)(l.gs - s.g_base) : 32};
-  const uint8_t *read = reads + l.rs, *win = genome + l.gs;
-  Extras x;
-  x.n = 0;
-  if (ODD && l.ok && !read_extras(R, D.nr, l.c.m, read, x)) {
-    st = 2;  // alphabet
-    l.ok = false;
-  }
-  const int m = l.ok ? l.c.m : 0, L = l.ok ? l.c.L : 0;
-  const MismatchRows M(slice, D, lane, k);
-  const Planes<ODD> P(slice, D, lane, k);
-  RW eq = 0;
-  if (ROWS) {
-    if (l.ok) eq = lane_rows<ODD>(R, W, l.c, read, win, x, D, M);
-  } else {
-    lane_planes<ODD>(R, D.nr, m, read, x, false, P.rd);
-    lane_planes<ODD>(W, D.nw, L, win, x, true, P.wn);
-  }
+  uint32_t eq = 0;
+  int st = odd ? diag_compare<ROWS, true>(g, s, D, lane, slice, l, eq)
+               : diag_compare<ROWS, false>(g, s, D, lane, slice, l, eq);
   __syncwarp();
-  {  // table and gap masks (adjacent) start from zero
-    const int end16 = D.table_bytes + D.masks_bytes;
-    for (int i = 16 * lane; i < end16; i += 512) sm_st128(table + i, Quad{0, 0, 0, 0});
-  }
+  const Sm table = slice + D.compare_bytes;
+  // table and gap masks (adjacent) start from zero
+  for (int i = 16 * lane; i < D.table_bytes + D.masks_bytes; i += 512)
+    sm_st128(table + i, Quad{0, 0, 0, 0});
   __syncwarp();
   end = WalkEnd{0, 0, 0, false};
-  const DiagTable T(table, D, lane, k);
-  if (l.ok) {
-    if (ROWS) st |= diag_lane<RW>(M, T, eq, D.reach, l, end, U, Lf);
-    else st |= diag_lane<RW>(P, T, (RW)P.matches(m, D.reach), D.reach, l, end, U, Lf);
+  const DiagTable T(table, lane, g.k);
+  if (!l.ok) return st;
+  if (ROWS)
+    return st | diag_lane<RW>(MismatchRows(slice, D, lane, g.k), T, (RW)eq, D.reach, l, end, U, Lf);
+  const int m = l.c.m;
+  if (odd) {
+    const Planes<true> P(slice, D, lane, g.k);
+    return st | diag_lane<RW>(P, T, (RW)P.matches(m, D.reach), D.reach, l, end, U, Lf);
   }
-  return st;
+  const Planes<false> P(slice, D, lane, g.k);
+  return st | diag_lane<RW>(P, T, (RW)P.matches(m, D.reach), D.reach, l, end, U, Lf);
 }
 
 // One warp tile; `next`: the tile after it (its offsets arrive while this
@@ -330,9 +343,9 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncwarp();
   if (fits) {
-    const Sm sr = slice + D.compare_bytes, sw = sr + 12 * D.rw;
-    odd = stream_planes(slice + D.raw, (int)(s.r_hi - s.r_base), sr, sr + 4 * D.rw, lane);
-    odd |= stream_planes(slice + (D.raw + D.src_r), (int)(s.g_hi - s.g_base), sw, sw + 4 * D.ww,
+    const Sm sr = slice + D.streams, sw = sr + 12 * D.rw;
+    odd = stream_planes(slice, (int)(s.r_hi - s.r_base), sr, sr + 4 * D.rw, lane);
+    odd |= stream_planes(slice + D.src_r, (int)(s.g_hi - s.g_base), sw, sw + 4 * D.ww,
                          lane);
   }
   const bool more = next < a.total_tiles;
@@ -355,7 +368,7 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
     if (!more || !fits_next) return;
     const Segment &h = a.segs[ahead.seg];
     const DiagLayout N = diag_layout(h.max_m, h.k, ROWS);
-    stage_tile(h, sn, slice + N.raw, slice + (N.raw + N.src_r), lane);
+    stage_tile(h, sn, slice, slice + N.src_r, lane);
   };
   if (!fits) {  // offsets no regular call can have: report, do not stage
     if (lane < count) g.scores[t0 + lane] = k + 1;
@@ -367,10 +380,8 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
   const GapMask U{masks}, Lf{masks + D.mwords * 128};
   __syncwarp();
   WalkEnd end;
-  if (__any_sync(0xffffffffu, odd != 0))
-    st |= diag_align<ROWS, true>(g.reads, g.genome, k, s, D, lane, slice, l, end, U, Lf);
-  else
-    st |= diag_align<ROWS, false>(g.reads, g.genome, k, s, D, lane, slice, l, end, U, Lf);
+  const bool any_odd = __any_sync(0xffffffffu, odd != 0);
+  st |= diag_align<ROWS>(g, s, D, any_odd, lane, slice, l, end, U, Lf);
   __syncwarp();
   prefetch();
   if (lane < count) g.scores[t0 + lane] = l.score;
@@ -438,7 +449,7 @@ __global__ void __launch_bounds__(128, kDiagCtas)
     const Segment &g = a.segs[now.seg];
     const DiagLayout D = diag_layout(g.max_m, g.k, ROWS);
     DiagSpan s;
-    const Sm raw = sm_at(slice) + D.raw;
+    const Sm raw = sm_at(slice);
     if (tile_span(a, now, 32, s)) stage_tile(g, s, raw, raw + D.src_r, lane);
   }
   while (now.tile < a.total_tiles) {

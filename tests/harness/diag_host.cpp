@@ -35,11 +35,11 @@ static int align(const TileArgs &a, const DiagSpan &s, const DiagLayout &D, Sm s
   using RW = typename DiagWord<ROWS>::type;
   int st = 0;
   RW eq[32] = {};
-  const Sm table = slice + D.compare_bytes, sr = table, sw = sr + 12 * D.rw;
+  const Sm table = slice + D.compare_bytes, sr = slice + D.streams, sw = sr + 12 * D.rw;
   if (ODD)
     for (int i = 0; i < 32; ++i) {
-      stream_odd(slice + D.raw, (int)(s.r_hi - s.r_base), sr + 8 * D.rw, i);
-      stream_odd(slice + (D.raw + D.src_r), (int)(s.g_hi - s.g_base), sw + 8 * D.ww, i);
+      stream_odd(slice, (int)(s.r_hi - s.r_base), sr + 8 * D.rw, i);
+      stream_odd(slice + D.src_r, (int)(s.g_hi - s.g_base), sw + 8 * D.ww, i);
     }
   for (int i = 0; i < 32; ++i) {
     DiagLane &l = ls[i];
@@ -66,7 +66,7 @@ static int align(const TileArgs &a, const DiagSpan &s, const DiagLayout &D, Sm s
   for (int i = 0; i < 32; ++i) {
     end[i] = WalkEnd{0, 0, 0, false};
     if (!ls[i].ok) continue;
-    const DiagTable T(table, D, i, a.k);
+    const DiagTable T(table, i, a.k);
     const MismatchRows M(slice, D, i, a.k);
     const Planes<ODD> P(slice, D, i, a.k);
     st |= ROWS ? lane<RW>(M, T, eq[i], D.reach, ls[i], end[i], U[i], Lf[i])
@@ -100,7 +100,7 @@ static int run(const TileArgs &a) {
       status |= 1;
       continue;
     }
-    const Sm sr = slice + D.compare_bytes, sw = sr + 12 * D.rw;
+    const Sm sr = slice + D.streams, sw = sr + 12 * D.rw;
     auto copy16 = [](Sm d, const uint8_t *p) { sm_st128(d, load16(p)); };
     auto stage = [&](int at) {
       for (int lane = 0; lane < 32; ++lane) {
@@ -109,14 +109,14 @@ static int run(const TileArgs &a) {
                     load16);
       }
     };
-    stage(D.raw);
+    stage(0);
     uint32_t odd = 0;
     DiagLane ls[32];
     WalkEnd end[32];
     GapMask U[32], Lf[32];
     for (int lane = 0; lane < 32; ++lane) {
-      odd |= stream_planes(slice + D.raw, (int)(s.r_hi - s.r_base), sr, sr + 4 * D.rw, lane);
-      odd |= stream_planes(slice + (D.raw + D.src_r), (int)(s.g_hi - s.g_base), sw,
+      odd |= stream_planes(slice, (int)(s.r_hi - s.r_base), sr, sr + 4 * D.rw, lane);
+      odd |= stream_planes(slice + D.src_r, (int)(s.g_hi - s.g_base), sw,
                            sw + 4 * D.ww, lane);
       const long t = t0 + lane < a.n ? t0 + lane : a.n - 1;
       if (!lane_candidate(s, lane && lane < count ? a.goff[t - 1] : s.g_lo, a.goff[t],

@@ -601,17 +601,19 @@ int upload(Lane &L, const saru_batch *b, saru_batch *db, bool copy = true) {
 }
 
 // The exact full-rectangle path on lane buffers (whole call).
-int run_full(Lane &L, const saru_batch *hb, const saru_batch *db, const Plan &pl,
-             const saru_result *dr) {
+int run_full(Lane &L, const saru_batch *hb, const saru_batch *db, const saru_result *dr) {
   const size_t n = (size_t)hb->n;
   int rc;
   std::vector<int64_t> eoff(n);
-  int64_t acc = 0;
+  int64_t acc = 0, min_m = INT32_MAX, max_m = 0, max_L = 0;
   for (size_t t = 0; t < n; ++t) {
     eoff[t] = acc;
     const int64_t L_ = (int64_t)hb->genome_offsets[t] - (t ? hb->genome_offsets[t - 1] : 0);
     const int64_t m_ = (int64_t)hb->read_offsets[t] - (t ? hb->read_offsets[t - 1] : 0);
     acc += (m_ + 1) * (L_ + 1);
+    min_m = std::min(min_m, m_);
+    max_m = std::max(max_m, m_);
+    max_L = std::max(max_L, L_);
   }
   if (acc > INT32_MAX) {
     set_error("call too large for the reference's int cell index (%lld cells)", (long long)acc);
@@ -635,6 +637,9 @@ int run_full(Lane &L, const saru_batch *hb, const saru_batch *db, const Plan &pl
   a.match = hb->match;
   a.mismatch = hb->mismatch;
   a.first_of_call = hb->first_of_call;
+  a.min_m = (int)min_m;
+  a.max_m = (int)max_m;
+  a.max_L = (int)max_L;
   a.genome_bytes = hb->genome_bytes;
   a.read_bytes = n ? hb->read_offsets[n - 1] : 0;
   a.arena = L.arena.as<short>();
@@ -642,7 +647,6 @@ int run_full(Lane &L, const saru_batch *hb, const saru_batch *db, const Plan &pl
   a.read_aln = reinterpret_cast<uint8_t *>(dr->read_aln);
   a.genome_aln = reinterpret_cast<uint8_t *>(dr->genome_aln);
   a.status = L.status.as<int>();
-  (void)pl;
   SARU_CUDA(saru::launch_full_kernels(a, s));
   g_launches.fetch_add(2);
   g_thread_launches += 2;
@@ -890,7 +894,7 @@ int align_host_impl(const saru_batch *b, saru_result *r, Lane &L, float *ms_out,
     }
   }
   if (full) {
-    if ((rc = run_full(L, b, &db, pl, &dr))) return rc;
+    if ((rc = run_full(L, b, &db, &dr))) return rc;
     SARU_CUDA(cudaMemcpyAsync(L.status_host, L.status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   }
   if (!copied && hc && !full) {  // banded, unsplit: the records

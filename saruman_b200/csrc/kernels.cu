@@ -10,15 +10,19 @@
 //  saru_band_kernel           the same for longer reads: bit-parallel banded
 //                             fill (saru_core.cuh) of 32- or 64-bit bands with
 //                             2-bit traceback decisions (band_tile.cuh).
-//  saru_full_fill_kernel      the exact full-rectangle path for inputs the
-//  saru_full_trace_kernel     banded kernel does not cover (other costs,
-//                             m <= 3k, k > 15, irregular windows): the
+//  saru_full_fill_rows_kernel the exact full-rectangle path for inputs the
+//  saru_full_fill_kernel      kernels above do not cover (other costs,
+//  saru_full_trace_kernel     m <= 3k, k > 15, irregular windows): the
 //                             reference's int16 recurrence over a device
-//                             arena holding every matrix of the call, then
-//                             its traceback over that arena.
+//                             arena holding every matrix of the call (rows in
+//                             shared memory; very short and very long reads
+//                             cell by cell), then its traceback over that
+//                             arena.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <stdlib.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "kernels.cuh"
@@ -506,6 +510,86 @@ __global__ void saru_full_fill_kernel(FullArgs a) {
   a.scores[t] = M[W * (L + 1) - 1];
 }
 
+// The same fill with the row above and the read in shared memory and the
+// cells written 16 bytes at a time: a matrix is one run of cells, a lane
+// shifts its cells into four registers and stores them at every 8th index of
+// the arena.  (The kernel above reads and writes each 2-byte cell in global
+// memory, a sector a lane: 631 us for 20k candidates of 36 bp, against 75.)
+// Bound by the serial chain along a row, a warp of 32 candidates and
+// (m + 1) x 64 + m x 32 bytes of shared memory each.
+struct CellRun {
+  short *to;     // the next cell
+  short *begin;  // the matrix
+  uint32_t a[4];
+  __device__ __forceinline__ void push(int v) {
+    a[0] = fshr32(a[0], a[1], 16);
+    a[1] = fshr32(a[1], a[2], 16);
+    a[2] = fshr32(a[2], a[3], 16);
+    a[3] = __byte_perm(a[3], (uint32_t)v, 0x5432);
+    ++to;
+    // (a block that begins before the matrix is its head, written apart)
+    if (((uintptr_t)to & 15u) == 0 && to - 8 >= begin)
+      *reinterpret_cast<uint4 *>(to - 8) = make_uint4(a[0], a[1], a[2], a[3]);
+  }
+  __device__ __forceinline__ void end() const {  // the cells past the last whole block
+    const int left = (int)(((uintptr_t)to >> 1) & 7u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i >= 8 - left) to[i - 8] = (short)(a[i >> 1] >> (16 * (i & 1)));
+  }
+};
+
+// PLAIN: no cell can leave 16 bits, so the reference's short arithmetic is
+// plain integer arithmetic.
+template <bool PLAIN>
+__global__ void __launch_bounds__(32) saru_full_fill_rows_kernel(FullArgs a) {
+  extern __shared__ uint4 smem_v[];
+  short *above = reinterpret_cast<short *>(smem_v) + threadIdx.x;  // column j at 32 * j
+  uint8_t *read = reinterpret_cast<uint8_t *>(smem_v) + 64L * (a.max_m + 1) + threadIdx.x;
+  const long t = 32L * blockIdx.x + threadIdx.x;
+  if (t >= a.n) return;
+  const long gs = gstart_of(a.goff, t), rs = t ? a.roff[t - 1] : 0;
+  const int m = (int)(a.roff[t] - rs), L = (int)(a.goff[t] - gs);
+  int so, eo;
+  flank_of(a.dirs[t], a.k, so, eo);
+  const uint8_t *g = a.genome + gs;
+  for (int j = 0; j < m; ++j) read[32 * j] = a.reads[rs + j];
+  auto cut = [](int v) { return PLAIN ? v : (int)(short)v; };
+  short *begin = a.arena + a.eoff[t];
+  // the matrix's cells before its first 16-byte block lie in row 0, column
+  // 0.. (m >= 7) or are written one by one with the whole matrix
+  CellRun run{begin, begin, {0, 0, 0, 0}};
+  const int head = (int)((8 - (((uintptr_t)begin >> 1) & 7u)) & 7u);
+  for (int j = 0; j < head; ++j) begin[j] = (short)j;
+  for (int j = 0; j <= m; ++j) {
+    above[32 * j] = (short)j;
+    run.push(j);
+  }
+  int first = 0;
+  for (int i = 0; i < L; ++i) {
+    if (i + 1 >= 2 * so + 1) first = cut(first + 1);
+    const uint8_t gi = g[i];
+    int left = first, diag = above[0];
+    above[0] = (short)first;
+    run.push(first);
+    auto cell = [&](int j, int corr) {
+      const int up = above[32 * (j + 1)];
+      const int d = cut(diag + (gi != read[32 * j] ? a.mismatch : a.match));
+      const int l = cut(left + a.mismatch);
+      const int u = cut(up + a.mismatch - corr);
+      left = min(min(d, u), l);
+      diag = up;
+      above[32 * (j + 1)] = (short)left;
+      run.push(left);
+    };
+#pragma unroll 4
+    for (int j = 0; j < m - 1; ++j) cell(j, 0);
+    cell(m - 1, i >= L - 2 * eo ? a.mismatch : 0);  // free steps down the last column
+    if (i == L - 1) a.scores[t] = left;
+  }
+  run.end();
+}
+
 __device__ __forceinline__ short arena_cell(const FullArgs &a, long P) { return a.arena[P]; }
 
 // The reference traceback (src/cuda-functions.cu:108-315) over the arena of
@@ -515,13 +599,13 @@ __global__ void saru_full_trace_kernel(FullArgs a) {
   if (t >= a.n) return;
   if (a.scores[t] > a.k) return;
   const long gs = gstart_of(a.goff, t), rs = t ? a.roff[t - 1] : 0;
-  const long m = a.roff[t] - rs, L = a.goff[t] - gs, W = m + 1;
+  const int m = (int)(a.roff[t] - rs), L = (int)(a.goff[t] - gs), W = m + 1;
   int so, eo;
   flank_of(a.dirs[t], a.k, so, eo);
-  const long base = a.eoff[t];
+  const int base = (int)a.eoff[t];  // cell indices fit 32 bits, as in the reference
   const long slot = gs + (long)a.k * t;
   const long slot_end = slot + L + a.k;
-  long P = base + (L + 1) * W - 1;
+  int P = base + (L + 1) * W - 1;
   long ap = slot;
   // the loop bound is on the absolute cell index, as in the reference
   while (P >= W) {
@@ -551,7 +635,7 @@ __global__ void saru_full_trace_kernel(FullArgs a) {
     if (ri >= 0 && ri < a.read_bytes) rch = a.reads[ri];
     else atomicOr(a.status, kStatusUndefined);
     uint8_t oa, ob;
-    long step;
+    int step;
     if (dg + a.mismatch == v) {
       oa = rch; ob = gch; step = W + 1;
     } else if (dg + a.match == v && gch == rch) {
@@ -617,6 +701,10 @@ cudaError_t allow_smem() {
     e = cudaFuncSetAttribute(saru_diag_kernel<true>, (cudaFuncAttribute)attr, most - 64);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(saru_diag_kernel<false>, (cudaFuncAttribute)attr, most - 64);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(saru_full_fill_rows_kernel<true>, (cudaFuncAttribute)attr, most);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(saru_full_fill_rows_kernel<false>, (cudaFuncAttribute)attr, most);
   if (e == cudaSuccess) g_attr_done |= 1ull << dev;
   return e;
 }
@@ -733,8 +821,24 @@ cudaError_t launch_full_kernels(const FullArgs &a, cudaStream_t s) {
   const int cta = 128;
   const unsigned grid = (unsigned)((a.n + cta - 1) / cta);
   if (grid == 0) return cudaSuccess;
-  saru_full_fill_kernel<<<grid, cta, 0, s>>>(a);
-  cudaError_t e = cudaGetLastError();
+  // the row above and the read of 32 candidates in shared memory: reads of 7
+  // bases (so that a matrix's head lies in row 0) up to 2.4 k (227 KB); others
+  // cell by cell in global memory
+  cudaError_t e = allow_smem();
+  if (e != cudaSuccess) return e;
+  const size_t rows = 64 * ((size_t)a.max_m + 1) + 32 * (size_t)a.max_m;
+  if (a.min_m >= 7 && rows <= (size_t)kMaxCtaSmem) {
+    // no cell leaves 16 bits if m + L + 2 steps of the larger cost do not
+    const long cost = std::max({1L, labs((long)a.match), labs((long)a.mismatch)});
+    const unsigned warps = (unsigned)((a.n + 31) / 32);
+    if (cost * ((long)a.max_m + a.max_L + 2) < 32767)
+      saru_full_fill_rows_kernel<true><<<warps, 32, rows, s>>>(a);
+    else
+      saru_full_fill_rows_kernel<false><<<warps, 32, rows, s>>>(a);
+  } else {
+    saru_full_fill_kernel<<<grid, cta, 0, s>>>(a);
+  }
+  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   saru_full_trace_kernel<<<grid, cta, 0, s>>>(a);
   return cudaGetLastError();

@@ -74,6 +74,7 @@ struct FullArgs {
   const int64_t *eoff;  // cell offset of each matrix in the arena
   long n;
   int k, match, mismatch, first_of_call;
+  int min_m, max_m, max_L;  // the shortest and longest read, the longest window
   long genome_bytes, read_bytes;
   short *arena;
   int32_t *scores;

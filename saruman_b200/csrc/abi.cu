@@ -653,8 +653,8 @@ int run_full(Lane &L, const saru_batch *hb, const saru_batch *db, const saru_res
   return SARU_OK;
 }
 
-// A call of at least 2 * kSplitMin candidates from host memory is split
-// into slices of whole tiles.  The copies in of every slice are issued
+// A call from host memory that makes two slices or more is split into
+// slices of whole tiles.  The copies in of every slice are issued
 // first (one event each), and the host's pass over the call (plan_host)
 // runs while they stream; then, for a banded call, the kernel of slice i
 // waits for its inputs and the copies out of slice i wait for its kernel,
@@ -665,12 +665,22 @@ int run_full(Lane &L, const saru_batch *hb, const saru_batch *db, const saru_res
 // launch makes; only candidate 0 of the call takes the first-of-call rule.
 // With pinned host buffers the copies run asynchronously; with pageable
 // ones they are correct but serialised.
-constexpr long kSplitMin = 1L << 18;
+//
+// A slice holds about kSliceBytes of inputs and slots, so that the first
+// kernel starts and the first results leave early, but no call has more than
+// kSplitParts slices (each costs nine calls into the driver).  176k
+// candidates of 100 bp (79 MB): 1.85 ms whole, 1.78 / 1.54 / 1.34 / 1.37 in
+// slices of 4 / 8 / 16 / 32 MB; 1.2M: 11.3 ms whole, 8.3 in slices of 16 MB.
+constexpr long kSliceBytes = 16L << 20;
 constexpr long kSplitParts = 32;
 
-long split_chunk(long n) {
-  const long c = ((n + kSplitParts - 1) / kSplitParts + 31) & ~31L;
-  return c < kSplitMin ? kSplitMin : c;
+long split_chunk(const saru_batch *b) {
+  const long n = b->n;
+  const double bytes = 2.0 * (double)b->genome_bytes + 2.0 * (double)b->total_slots;
+  long least = n;  // (sizes that make no sense are refused later)
+  if (bytes > 0) least = (long)std::min((double)n, (double)kSliceBytes / bytes * (double)n);
+  const long c = std::max({(n + kSplitParts - 1) / kSplitParts, least, 4096L});
+  return (c + 31) & ~31L;
 }
 
 // The slice edges of a large call, checked before its copies are issued:
@@ -812,8 +822,8 @@ int align_host_impl(const saru_batch *b, saru_result *r, Lane &L, float *ms_out,
                     const HostCompact *hc = nullptr) {
   Plan pl;
   int rc;
-  const bool big = b->n >= 2 * kSplitMin && b->k >= 0;
-  const long chunk = big ? split_chunk(b->n) : 0;
+  const long chunk = b->n > 0 && b->k >= 0 ? split_chunk(b) : 0;
+  const bool big = chunk > 0 && b->n >= 2 * chunk;
   if (!big && (rc = plan_host(b, &pl))) return rc;
   if (big && (rc = check_slice_edges(b, chunk))) return rc;
   const int dev = current_device();

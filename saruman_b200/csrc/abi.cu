@@ -666,21 +666,24 @@ int run_full(Lane &L, const saru_batch *hb, const saru_batch *db, const saru_res
 // With pinned host buffers the copies run asynchronously; with pageable
 // ones they are correct but serialised.
 //
-// A slice holds about kSliceBytes of inputs and slots, so that the first
-// kernel starts and the first results leave early, but no call has more than
-// kSplitParts slices (each costs nine calls into the driver).  176k
+// A slice holds up to kSliceBytes of inputs and slots, so that the first
+// kernel starts and the first results leave early: a power of two of
+// candidates, at most kSplitMost; a call of more than kSplitParts such slices
+// has kSplitParts larger ones (each costs nine calls into the driver).  176k
 // candidates of 100 bp (79 MB): 1.85 ms whole, 1.78 / 1.54 / 1.34 / 1.37 in
 // slices of 4 / 8 / 16 / 32 MB; 1.2M: 11.3 ms whole, 8.3 in slices of 16 MB.
 constexpr long kSliceBytes = 16L << 20;
+constexpr long kSplitMost = 1L << 18;
 constexpr long kSplitParts = 32;
 
 long split_chunk(const saru_batch *b) {
   const long n = b->n;
   const double bytes = 2.0 * (double)b->genome_bytes + 2.0 * (double)b->total_slots;
-  long least = n;  // (sizes that make no sense are refused later)
-  if (bytes > 0) least = (long)std::min((double)n, (double)kSliceBytes / bytes * (double)n);
-  const long c = std::max({(n + kSplitParts - 1) / kSplitParts, least, 4096L});
-  return (c + 31) & ~31L;
+  // (sizes that make no sense are refused later)
+  const double fit = bytes > 0 ? (double)kSliceBytes / bytes * (double)n : (double)kSplitMost;
+  long c = 4096;
+  while (c < kSplitMost && (2.0 * (double)c <= fit || c * kSplitParts < n)) c *= 2;
+  return std::max(c, ((n + kSplitParts - 1) / kSplitParts + 31) & ~31L);
 }
 
 // The slice edges of a large call, checked before its copies are issued:

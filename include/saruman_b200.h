@@ -173,20 +173,17 @@ int saru_align_device(const saru_batch *batch, saru_result *result, void *scratc
  * forbids other allocations, or a code path that must not add an
  * allocation's synchronisation and latency.  No counterpart in the
  * reference.  Same batch, result and stream arguments and the same outputs
- * as saru_align_device; the banded kernel's scratch comes from a device
- * array inside the library of SARU_STATIC_SCRATCH_BYTES (32 MiB), present on
- * every GPU that loads the library until the process exits.  Fewer thread
- * blocks run when the planes of a full grid do not fit in the array.  A batch outside the banded kernel's domain
- * is refused with SARU_E_INVALID and a message; so would be one that cannot
- * get a single block, which with reads of at most 512 bases (about 0.5 MB
- * of planes a block) cannot happen at this array size.  The first call on a
+ * as saru_align_device; the kernel's scratch (its tile counter) comes from a
+ * device array inside the library of SARU_STATIC_SCRATCH_BYTES (32 MiB),
+ * present on every GPU that loads the library until the process exits.  A
+ * batch outside the kernel's domain is refused with SARU_E_INVALID and a
+ * message.  The first call on a
  * device looks up the array's device address (cudaGetSymbolAddress, with
  * that device current), so make that first call before any stream capture;
  * the address is kept for the life of the process, so a cudaDeviceReset
  * after that first call is not supported.  All calls share the array: each
- * call clears the work counter at its start and writes every other byte it
- * reads, so nothing from an earlier call is used, but calls that overlap on
- * the GPU race. */
+ * call clears the work counter at its start, so nothing from an earlier call
+ * is used, but calls that overlap on the GPU race. */
 #define SARU_STATIC_SCRATCH_BYTES (32u << 20)
 int saru_align_device_static(const saru_batch *batch, saru_result *result, void *stream);
 
@@ -195,7 +192,8 @@ int saru_align_device_static(const saru_batch *batch, saru_result *result, void 
  * installs the fastest here; every entry point that launches the banded
  * kernel for that class (saru_scratch_bytes included) then uses it.  0 in
  * a field keeps the default: as many warps per CTA (up to 4) and CTAs per
- * SM as fit, 32-bit band words when k <= 7 and 64-bit ones above.  A
+ * SM as fit.  word_bits sizes the scratch only (32-bit band words when
+ * k <= 7 and 64-bit ones above by default).  A
  * multi-call launch looks up its class by (longest read, largest k).
  * Results do not depend on the shape.  Not in the reference. */
 typedef struct {

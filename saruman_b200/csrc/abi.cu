@@ -356,8 +356,7 @@ using saru::CompactOut;
 // t0 > 0 (a multiple of 32, one call): align candidates t0 .. n - 1 only.
 int run_band_multi(const saru_batch *calls, const saru_result *res, int ncalls, const Plan &pl,
                    void *scratch, size_t scratch_bytes, int *status_dev, int dev,
-                   cudaStream_t s, long max_grid = 0, const CompactOut *cmp = nullptr,
-                   long t0 = 0) {
+                   cudaStream_t s, const CompactOut *cmp = nullptr, long t0 = 0) {
   if (ncalls < 1 || ncalls > saru::kMaxSegs) {
     set_error("%d calls in one launch (1..%d)", ncalls, saru::kMaxSegs);
     return SARU_E_INVALID;
@@ -406,37 +405,29 @@ int run_band_multi(const saru_batch *calls, const saru_result *res, int ncalls, 
     g.k = b->k;
     g.max_m = b->max_read_length;
     g.first_of_call = b->first_of_call;
-    g.wide = (b->k > 7 && (ncalls > 1 || pl.wide)) || tn.word_bits == 64;
     tiles += (b->n - g.t0 + 31) / 32;
     total_n += b->n - g.t0;
-    wide_any |= g.wide;
+    wide_any |= (b->k > 7 && (ncalls > 1 || pl.wide)) || tn.word_bits == 64;
   }
   if (tiles == 0) return SARU_OK;
   a.total_tiles = tiles;
   a.max_m = max_m;
   a.max_k = max_k;
-  a.wide_any = wide_any;
   a.warps_req = tn.warps;
-  a.grid = saru::band_grid(sm_count(dev), total_n,
-                           saru::band_layout(max_m, max_k, tn.warps, wide_any != 0),
-                           smem_per_sm(dev), tn.ctas_per_sm);
-  if (max_grid > 0 && a.grid > max_grid) a.grid = max_grid;
-  const size_t need = saru::band_scratch_bytes(a.grid, max_m, max_k, wide_any != 0, tn.warps);
+  const long grid = saru::band_grid(sm_count(dev), total_n,
+                                    saru::band_layout(max_m, max_k, tn.warps, wide_any != 0),
+                                    smem_per_sm(dev), tn.ctas_per_sm);
+  const size_t need = saru::band_scratch_bytes(grid, max_m, max_k, wide_any != 0, tn.warps);
   if (need > scratch_bytes) {
     set_error("scratch too small: %zu < %zu", scratch_bytes, need);
     return SARU_E_INVALID;
   }
-  if (reinterpret_cast<uintptr_t>(scratch) & 15u) {  // the kernel copies 16-byte plane pairs
+  if (reinterpret_cast<uintptr_t>(scratch) & 15u) {
     set_error("scratch must be 16-byte aligned");
     return SARU_E_INVALID;
   }
   a.counter = reinterpret_cast<int *>(scratch);
-  a.planes = reinterpret_cast<uint8_t *>(scratch) + saru::kCounterBytes;
-  if (saru::diag_launch(max_m)) {
-    SARU_CUDA(saru::launch_diag_kernel(a, sm_count(dev), smem_per_sm(dev), tn.ctas_per_sm, s));
-  } else {
-    SARU_CUDA(saru::launch_band_kernel(a, s));
-  }
+  SARU_CUDA(saru::launch_diag_kernel(a, sm_count(dev), smem_per_sm(dev), tn.ctas_per_sm, s));
   g_launches.fetch_add(1);
   g_thread_launches += 1;
   return SARU_OK;
@@ -545,7 +536,7 @@ int run_band_classes(const saru_batch *calls, const saru_result *res, int ncalls
     }
     return run_band_multi(cb.data(), cr.data(), (int)cb.size(), pl,
                           static_cast<uint8_t *>(scratch) + L.scratch_off, L.scratch_bytes,
-                          status_dev, dev, st, 0, cmp ? cc.data() : nullptr);
+                          status_dev, dev, st, cmp ? cc.data() : nullptr);
   };
   if (cls.size() == 1) return launch(cls[0], s);
   if (dev < 0 || dev >= 64) return SARU_E_INVALID;
@@ -565,12 +556,11 @@ int run_band_classes(const saru_batch *calls, const saru_result *res, int ncalls
 
 int run_band(const saru_batch *b, const Plan &pl, const saru_result *r, void *scratch,
              size_t scratch_bytes, int *status_dev, int dev, cudaStream_t s,
-             long max_grid = 0, const CompactOut *cmp = nullptr, long t0 = 0) {
+             const CompactOut *cmp = nullptr, long t0 = 0) {
   if (b->n == 0) return SARU_OK;
   saru_batch one = *b;
   one.max_read_length = pl.max_m;
-  return run_band_multi(&one, r, 1, pl, scratch, scratch_bytes, status_dev, dev, s, max_grid,
-                        cmp, t0);
+  return run_band_multi(&one, r, 1, pl, scratch, scratch_bytes, status_dev, dev, s, cmp, t0);
 }
 
 // Host batch -> device buffers of `lane`, returns device-side view (with
@@ -788,7 +778,7 @@ int band_slices(Lane &L, const saru_batch *b, int m0, const saru_batch &db,
     SARU_CUDA(cudaStreamWaitEvent(sr, L.ev_in[(size_t)i], 0));
     saru_batch slice = db;
     slice.n = (int32_t)t1;
-    if ((rc = run_band(&slice, pl, &dr, L.scratch.p, L.scratch.n, L.status.as<int>(), dev, sr, 0,
+    if ((rc = run_band(&slice, pl, &dr, L.scratch.p, L.scratch.n, L.status.as<int>(), dev, sr,
                        hc ? &dcmp : nullptr, t0)))
       return rc;
     SARU_CUDA(cudaEventRecord(L.ev_run, sr));
@@ -892,7 +882,7 @@ int align_host_impl(const saru_batch *b, saru_result *r, Lane &L, float *ms_out,
     }
     const long grid = band_grid(dev, b->n, pl.max_m, b->k);
     if ((rc = L.scratch.ensure(band_scratch_bytes(grid, pl.max_m, b->k, pl.wide)))) return rc;
-    if ((rc = run_band(&db, pl, &dr, L.scratch.p, L.scratch.n, L.status.as<int>(), dev, s, 0,
+    if ((rc = run_band(&db, pl, &dr, L.scratch.p, L.scratch.n, L.status.as<int>(), dev, s,
                        hc ? &dcmp : nullptr)))
       return rc;
     SARU_CUDA(cudaMemcpyAsync(L.status_host, L.status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1258,18 +1248,10 @@ int saru_align_device_static(const saru_batch *batch, saru_result *result, void 
   pl.band = true;
   pl.max_m = batch->max_read_length;
   pl.wide = batch->k > 7;
-  // as many persistent CTAs as the array holds planes for (each CTA's warps
-  // need their own slice); a batch that cannot get even one CTA is refused
-  const size_t per_cta = band_scratch_bytes(1, pl.max_m, batch->k, pl.wide);
-  const long max_grid = (long)(kStaticScratchBytes / (per_cta ? per_cta : 1));
-  if (max_grid < 1) {
-    set_error("saru_align_device_static: one thread block needs %zu bytes of scratch, the "
-              "static array holds %zu",
-              per_cta, kStaticScratchBytes);
-    return SARU_E_INVALID;
-  }
-  return run_band(batch, pl, result, scratch, kStaticScratchBytes, result->status, dev,
-                  reinterpret_cast<cudaStream_t>(stream), max_grid);
+  // (the array holds all the kernel uses, whatever a caller's scratch of this
+  // batch would have to be)
+  return run_band(batch, pl, result, scratch, SIZE_MAX, result->status, dev,
+                  reinterpret_cast<cudaStream_t>(stream));
 }
 
 int64_t saru_compact_record_bytes(int32_t max_read_length, int32_t k) {
@@ -1302,7 +1284,7 @@ int saru_align_device_compact(const saru_batch *batch, int32_t *scores, uint8_t 
   const saru_result r{scores, nullptr, nullptr, status};
   const CompactOut cmp{records, (long)record_bytes};
   return run_band(batch, pl, &r, scratch, scratch_bytes, status, dev,
-                  reinterpret_cast<cudaStream_t>(stream), 0, &cmp);
+                  reinterpret_cast<cudaStream_t>(stream), &cmp);
 }
 
 int saru_align_multi_device_compact(const saru_batch *calls, saru_result *results,

@@ -25,8 +25,16 @@
 
 namespace saru {
 
-// Columns are kept as bytes, so reads up to this length.
-constexpr int kDiagMaxM = 255;
+// A table cell holds a column + 1: a byte for reads up to 255 bases, two for
+// longer ones.
+constexpr int kByteColumns = 255;
+
+// The forms a launch runs in: `rows` or planes (DiagLayout), bytes a cell.
+template <bool ROWS_, int CELL_>
+struct DiagForm {
+  static constexpr bool ROWS = ROWS_;
+  static constexpr int CELL = CELL_;
+};
 
 struct alignas(16) Quad {
   uint32_t x, y, z, w;
@@ -111,6 +119,11 @@ __device__ __forceinline__ int sm_ld8(Sm p) {
   asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(p.a));
   return (int)v;
 }
+__device__ __forceinline__ int sm_ld16(Sm p) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(p.a));
+  return (int)v;
+}
 __device__ __forceinline__ uint32_t sm_ld32(Sm p) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(p.a));
@@ -144,6 +157,7 @@ __device__ __forceinline__ int sm_low(Sm p, int bits) { return (int)(p.a & (uint
 #else
 inline Sm sm_at(void *p) { return Sm{static_cast<uint8_t *>(p)}; }
 inline int sm_ld8(Sm p) { return *p.a; }
+inline int sm_ld16(Sm p) { return *reinterpret_cast<uint16_t *>(p.a); }
 inline uint32_t sm_ld32(Sm p) { return *reinterpret_cast<uint32_t *>(p.a); }
 inline Quad sm_ld128(Sm p) { return *reinterpret_cast<Quad *>(p.a); }
 inline void sm_st8(Sm p, int v) { *p.a = (uint8_t)v; }
@@ -168,7 +182,7 @@ SARU_HD int low_bit(uint64_t x) {
 // ---------------------------------------------------------------------------
 //
 //   [compare: what a lane looks its mismatches up in, see below]
-//   [table: 32 bytes per diagonal and level, see DiagTable]
+//   [table: 32 cells per diagonal and level, see DiagTable]
 //   [gap masks: 2 x mwords x 32 words, and a word more]
 // The tile's bytes lie over the front of the first two and their bit streams
 // at the end of them until the compare part is made; after the walk the bytes
@@ -201,7 +215,7 @@ SARU_HD int table_cells(int e, int k) {
   return x * (2 * k + 4 + x) + (e - x) * (3 * k + 5);
 }
 
-SARU_HD DiagLayout diag_layout(int max_m, int k, bool rows) {
+SARU_HD DiagLayout diag_layout(int max_m, int k, bool rows, int cell) {
   DiagLayout D;
   D.reach = 5 * k / 2;
   D.diags = (k + D.reach + 2) & ~1;
@@ -217,7 +231,7 @@ SARU_HD DiagLayout diag_layout(int max_m, int k, bool rows) {
   D.compare_bytes =
       rows ? (D.diags * D.nr + 2) * 128 : (D.nr + D.nw + 2) * 512;
   const int streams = up16(3 * 4 * (D.rw + D.ww));
-  D.table_bytes = table_cells(k > 0 ? k : 1, k) * 32;
+  D.table_bytes = table_cells(k > 0 ? k : 1, k) * 32 * cell;
   D.masks_bytes = (2 * D.mwords + 1) * 128;
   int front = D.compare_bytes + D.table_bytes;
   const int raw = D.src_r + D.src_w;
@@ -529,12 +543,19 @@ SARU_HD void lane_planes(const StreamWords &s, int entries, int len, const uint8
 // The table of one lane, levels 0 .. k - 1: at(e, d) is 1 + the furthest
 // column of diagonal d with a value <= e, 0 if none is known; columns end at
 // m - 1 (the last one has rules of its own).
+template <int CELL>
 struct DiagTable {
+  static constexpr int kStep = 32 * CELL;  // bytes from a diagonal to the next
   Sm base;  // diagonal 0 of level 0
   int k;
-  SARU_HD DiagTable(Sm table, int lane, int k_) : base(table + (lane + 64)), k(k_) {}
-  SARU_HD Sm cell(int e, int d) const { return base + (table_cells(e, k) + e + d) * 32; }
-  SARU_HD int at(int e, int d) const { return sm_ld8(cell(e, d)); }
+  SARU_HD DiagTable(Sm table, int lane, int k_) : base(table + (lane * CELL + 2 * kStep)), k(k_) {}
+  SARU_HD Sm cell(int e, int d) const { return base + (table_cells(e, k) + e + d) * kStep; }
+  static SARU_HD int get(Sm c) { return CELL == 1 ? sm_ld8(c) : sm_ld16(c); }
+  static SARU_HD void put(Sm c, int s) {
+    if (CELL == 1) sm_st8(c, s);
+    else sm_st16(c, (uint32_t)s);
+  }
+  SARU_HD int at(int e, int d) const { return get(cell(e, d)); }
   // whether level e has a cell for d
   SARU_HD bool has(int e, int d) const {
     const int hi = 2 * k + e < 3 * k - e ? 2 * k + e : 3 * k - e;
@@ -584,8 +605,9 @@ struct DiagExit {
 // At 100 bp and k = 5 a candidate has 36 cells (so = 0) or 78 against 100
 // columns of about 85 instructions (fill, decisions, walk) of the banded
 // form.
-template <typename RW, class X>
-SARU_HD DiagExit lane_levels(const Cand &c, const X &P, const DiagTable &T, RW eq, int reach) {
+template <typename RW, class X, class Table>
+SARU_HD DiagExit lane_levels(const Cand &c, const X &P, const Table &T, RW eq, int reach) {
+  constexpr int N = Table::kStep;
   const int k = c.k, m = c.m;
   DiagExit x;
   x.score = k + 1;
@@ -619,13 +641,13 @@ SARU_HD DiagExit lane_levels(const Cand &c, const X &P, const DiagTable &T, RW e
     auto keep = [&](Sm to, int s) {
       if (!X::kStops) s = s < m ? s : m;
       short_of = push_sign(short_of, s - m);
-      if (e < k) sm_st8(to, s);
+      if (e < k) Table::put(to, s);
     };
     // a level has an odd number of diagonals: one, then fours and a pair, so
     // that one's loads cover the others'
-    int pm = sm_ld8(prev), p0 = sm_ld8(prev + 32);
+    int pm = Table::get(prev), p0 = Table::get(prev + N);
     {
-      int s = start(sm_ld8(prev + -32), pm, p0);
+      int s = start(Table::get(prev + -N), pm, p0);
       const int f = bfind32(P.window(s, row));
       s += 31 - f;
       if (f < 0) extend(s, f, row);
@@ -633,10 +655,10 @@ SARU_HD DiagExit lane_levels(const Cand &c, const X &P, const DiagTable &T, RW e
     }
     int left = hi - lo;
     for (; left >= 4; left -= 4) {
-      prev = prev + 128;
-      cur = cur + 128;
-      const int p1 = sm_ld8(prev + -64), p2 = sm_ld8(prev + -32), p3 = sm_ld8(prev),
-                p4 = sm_ld8(prev + 32);
+      prev = prev + 4 * N;
+      cur = cur + 4 * N;
+      const int p1 = Table::get(prev + -2 * N), p2 = Table::get(prev + -N), p3 = Table::get(prev),
+                p4 = Table::get(prev + N);
       int sa = start(pm, p0, p1), sb = start(p0, p1, p2), sc = start(p1, p2, p3),
           sd = start(p2, p3, p4);
       const typename X::Row r1 = P.next(row), r2 = P.next(r1), r3 = P.next(r2), r4 = P.next(r3);
@@ -652,16 +674,16 @@ SARU_HD DiagExit lane_levels(const Cand &c, const X &P, const DiagTable &T, RW e
         extend(sc, fc, r3);
         extend(sd, fd, r4);
       }
-      keep(cur + -96, sa);
-      keep(cur + -64, sb);
-      keep(cur + -32, sc);
+      keep(cur + -3 * N, sa);
+      keep(cur + -2 * N, sb);
+      keep(cur + -N, sc);
       keep(cur, sd);
       pm = p3;
       p0 = p4;
       row = r4;
     }
     if (left) {
-      const int p1 = sm_ld8(prev + 64), p2 = sm_ld8(prev + 96);
+      const int p1 = Table::get(prev + 2 * N), p2 = Table::get(prev + 3 * N);
       int sa = start(pm, p0, p1), sb = start(p0, p1, p2);
       const typename X::Row r1 = P.next(row), r2 = P.next(r1);
       const int fa = bfind32(P.window(sa, r1)), fb = bfind32(P.window(sb, r2));
@@ -671,8 +693,8 @@ SARU_HD DiagExit lane_levels(const Cand &c, const X &P, const DiagTable &T, RW e
         extend(sa, fa, r1);
         extend(sb, fb, r2);
       }
-      keep(cur + 32, sa);
-      keep(cur + 64, sb);
+      keep(cur + N, sa);
+      keep(cur + 2 * N, sb);
     }
     const RW R = (RW)((RW)~short_of & lowmask<RW>(hi - lo + 1)) << (RW)(reach - hi);
     // the last column: a row has value <= e by a diagonal step (a mismatch
@@ -766,8 +788,8 @@ SARU_HD int first_column(const X &P, int so, int i) {
 // to the furthest cell of value v - 1, whichever comes first: at most
 // 2 v + 1 rounds.  The borders follow the reference's rules (saru_core.cuh,
 // traceback_band).
-template <typename RW, class X>
-SARU_HD WalkEnd lane_diag_walk(const Cand &c, const X &P, const DiagTable &T, const DiagExit &x,
+template <typename RW, class X, class Table>
+SARU_HD WalkEnd lane_diag_walk(const Cand &c, const X &P, const Table &T, const DiagExit &x,
                                RW eq, int reach, const GapMask &U, const GapMask &Lf) {
   const int m = c.m, so = c.so, k = c.k;
   int nup = x.ups, d = x.d, v = x.v, col = m;

@@ -1,15 +1,12 @@
 // kernels.cu -- sm_100a kernels of the alignment stage.
 //
-//  saru_diag_kernel           the production path for reads up to 255 bases:
-//                             persistent warps over 32-candidate tiles (one
-//                             lane per candidate), furthest columns by
+//  saru_diag_kernel           the production path (reads up to 512 bases, k up
+//                             to 15): persistent warps over 32-candidate tiles
+//                             (one lane per candidate), furthest columns by
 //                             diagonal and error count (diag_tile.cuh),
 //                             traceback and slot strings or compact records
 //                             on the device; a launch covers segments (calls,
 //                             or slices [t0, t1) of one call).
-//  saru_band_kernel           the same for longer reads: bit-parallel banded
-//                             fill (saru_core.cuh) of 32- or 64-bit bands with
-//                             2-bit traceback decisions (band_tile.cuh).
 //  saru_full_fill_rows_kernel the exact full-rectangle path for inputs the
 //  saru_full_fill_kernel      kernels above do not cover (other costs,
 //  saru_full_trace_kernel     m <= 3k, k > 15, irregular windows): the
@@ -33,135 +30,6 @@
 namespace saru {
 
 __device__ __forceinline__ long gstart_of(const int32_t *goff, long t) { return t ? goff[t - 1] : 0; }
-
-// ---------------------------------------------------------------------------
-// banded kernel: persistent warps over warp tiles (band_tile.cuh)
-// ---------------------------------------------------------------------------
-
-// One warp tile of one segment (the phases of band_tile.cuh).
-template <typename T>
-__device__ __forceinline__ int band_tile(const TileArgs &ta, long wt, int lane, uint8_t *st_reads,
-                                         uint8_t *st_win, uint8_t *region, void *planes_v,
-                                         long pslot) {
-  // this lane's plane units: unit u at lane_units + u * row_bytes (a unit
-  // row of the whole grid's lanes is a few MB, so the offset of a unit is a
-  // 32-bit product widened by one multiply-add)
-  uint8_t *lane_units = reinterpret_cast<uint8_t *>(planes_v) + pslot * kPlaneUnit;
-  const uint32_t row_bytes = (uint32_t)(ta.pstride * kPlaneUnit);
-  auto pair_at = [&](int j) -> PlanePair<T> * {
-    return reinterpret_cast<PlanePair<T> *>(
-        lane_units + (unsigned long long)(uint32_t)plane_unit_of<T>(j) * row_bytes +
-        plane_half_of<T>(j));
-  };
-  uint32_t *region32 = reinterpret_cast<uint32_t *>(region);
-  auto ld16 = [](uint8_t *d, const uint8_t *g) {
-    *reinterpret_cast<uint4 *>(d) = __ldg(reinterpret_cast<const uint4 *>(g));
-  };
-  auto ld1 = [](const uint8_t *g) -> uint8_t { return __ldg(g); };
-  auto st16 = [](uint8_t *g, const uint8_t *d) {
-    *reinterpret_cast<uint4 *>(g) = *reinterpret_cast<const uint4 *>(d);
-  };
-  const TileSpan s = tile_span(ta, wt);
-  if (!s.fits) {  // offsets no regular call can have: report, do not stage
-    const long t = s.t0 + lane;
-    if (t < ta.n) ta.scores[t] = ta.k + 1;
-    return 1;
-  }
-  stage_in(st_reads, ta.reads, s.r_lo, s.r_hi, s.r_base, lane, ld16, ld1);
-  stage_in(st_win, ta.genome, s.g_lo, s.g_hi, s.g_base, lane, ld16, ld1);
-  __syncwarp();
-  LaneState ls;
-  int st = lane_fill<T>(
-      ta, s, lane, st_reads, st_win, region32, ls,
-      plane_writer<T>(
-          [&](long u, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-            *reinterpret_cast<uint4 *>(lane_units + (unsigned long long)(uint32_t)u * row_bytes) =
-                make_uint4(x, y, z, w);
-          }));
-  __syncwarp();
-  // the traceback walk's plane ring in the region: asynchronous 8- or
-  // 16-byte copies from the plane scratch, one copy group per column
-  const auto ring = plane_ring<T>(
-      reinterpret_cast<PlanePair<T> *>(region) + lane,
-      [&](PlanePair<T> *dst, int j) {
-        const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-        const size_t g = __cvta_generic_to_global(pair_at(j));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(g),
-                     "n"((int)sizeof(PlanePair<T>))
-                     : "memory");
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-      },
-      [] { asm volatile("cp.async.wait_group %0;\n" ::"n"(kRing - 1) : "memory"); });
-  if (ta.records) {  // compact records straight to global memory
-    uint32_t *rec = reinterpret_cast<uint32_t *>(ta.records + (s.t0 + lane) * ta.rec_bytes);
-    st |= lane_traceback_ops<T>(ta, s, lane, ls, ring, [&](int w, uint32_t v) { rec[w] = v; });
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncwarp();
-    return st;
-  }
-  uint32_t up_r[kMaxGapRuns], left_r[kMaxGapRuns];
-  LaneWalk w;
-  st |= lane_traceback_walk<T>(ta, s, lane, ls, ring, up_r, left_r, w);
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  __syncwarp();
-  uint8_t *out_r = region;
-  uint8_t *out_g = region + s.o_span_r;
-  const long out_bytes = out_area_bytes(ta.max_m, ta.k);
-  {
-    uint4 *p4 = reinterpret_cast<uint4 *>(region);
-    const long nv = out_bytes >> 4;
-    for (long i = lane; i < nv; i += 32) p4[i] = make_uint4(0, 0, 0, 0);
-  }
-  __syncwarp();
-  lane_write_strings(ta, s, lane, st_reads, st_win, out_r, out_g, ls, w);
-  __syncwarp();
-  stage_out(ta.read_aln, out_r, s.s_lo, s.s_hi, s.o_base_r, lane, st16);
-  stage_out(ta.genome_aln, out_g, s.s_lo, s.s_hi, s.o_base_g, lane, st16);
-  __syncwarp();
-  return st;
-}
-
-// Persistent warps take 32-candidate tiles from a launch-wide counter; a
-// tile belongs to one segment (a call with its own m, k and band width).
-// The bounds hold the kernel to 128 registers a thread: above that an SM
-// sub-partition's register file holds 3 of these warps instead of 4.
-__global__ void __launch_bounds__(128, 4) saru_band_kernel(const __grid_constant__ KernelArgs a) {
-  extern __shared__ uint4 smem_v[];
-  const int lane = threadIdx.x & 31;
-  const int wid = threadIdx.x >> 5;
-  const int WARPS = blockDim.x >> 5;
-  uint8_t *ws = reinterpret_cast<uint8_t *>(smem_v) + (long)wid * a.warp_smem;
-  uint8_t *st_reads = ws;
-  uint8_t *st_win = ws + a.rs_bytes;
-  uint8_t *region = st_win + a.ws_bytes;
-  const long gwarp = (long)blockIdx.x * WARPS + wid;
-  const long pstride = (long)gridDim.x * WARPS * 32;
-  const long pslot = gwarp * 32 + lane;
-  for (;;) {
-    int tile = 0;
-    if (lane == 0) tile = atomicAdd(a.counter, 1);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if (tile >= a.total_tiles) break;
-    int lo = 0, hi = a.nseg - 1;  // last segment with tile_begin <= tile
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (a.segs[mid].tile_begin <= tile) lo = mid;
-      else hi = mid - 1;
-    }
-    const Segment &g = a.segs[lo];
-    const TileArgs ta{g.genome, g.reads, g.goff, g.roff, g.dirs, g.n, g.k, g.max_m,
-                      g.first_of_call, g.scores, g.read_aln, g.genome_aln, a.planes, pstride,
-                      a.rs_bytes, a.ws_bytes, a.warp_smem - a.rs_bytes - a.ws_bytes,
-                      g.records, g.rec_bytes, g.t0};
-    const long wt = tile - g.tile_begin;
-    int status = g.wide ? band_tile<uint64_t>(ta, wt, lane, st_reads, st_win, region, a.planes, pslot)
-                        : band_tile<uint32_t>(ta, wt, lane, st_reads, st_win, region, a.planes, pslot);
-    status = __reduce_or_sync(0xffffffffu, status);
-    if (status && lane == 0)
-      atomicOr(g.status, (status & 1 ? kStatusIrregular : 0) | (status & 2 ? kStatusAlphabet : 0) |
-                             (status & 4 ? kStatusOverflow : 0));
-  }
-}
 
 // ---------------------------------------------------------------------------
 // diagonal kernel: persistent warps over warp tiles (diag_tile.cuh)
@@ -278,8 +146,8 @@ __device__ __forceinline__ int diag_compare(const Segment &g, const DiagSpan &s,
 }
 
 // Levels and walk of a lane on its mismatch look-up P.
-template <typename RW, class X>
-__device__ __forceinline__ int diag_lane(const X &P, const DiagTable &T, RW eq, int reach,
+template <typename RW, class X, class Table>
+__device__ __forceinline__ int diag_lane(const X &P, const Table &T, RW eq, int reach,
                                          DiagLane &l, WalkEnd &end, const GapMask &U,
                                          const GapMask &Lf) {
   const DiagExit x = lane_levels<RW>(l.c, P, T, eq, reach);
@@ -292,10 +160,11 @@ __device__ __forceinline__ int diag_lane(const X &P, const DiagTable &T, RW eq, 
 }
 
 // From the tile's bit streams to the lanes' walks.
-template <bool ROWS>
+template <class F>
 __device__ __forceinline__ int diag_align(const Segment &g, const DiagSpan &s, const DiagLayout &D,
                                           bool odd, int lane, Sm slice, DiagLane &l, WalkEnd &end,
                                           const GapMask &U, const GapMask &Lf) {
+  constexpr bool ROWS = F::ROWS;
   using RW = typename DiagWord<ROWS>::type;
   uint32_t eq = 0;
   int st = odd ? diag_compare<ROWS, true>(g, s, D, lane, slice, l, eq)
@@ -307,7 +176,7 @@ __device__ __forceinline__ int diag_align(const Segment &g, const DiagSpan &s, c
     sm_st128(table + i, Quad{0, 0, 0, 0});
   __syncwarp();
   end = WalkEnd{0, 0, 0, false};
-  const DiagTable T(table, lane, g.k);
+  const DiagTable<F::CELL> T(table, lane, g.k);
   if (!l.ok) return st;
   if (ROWS)
     return st | diag_lane<RW>(MismatchRows(slice, D, lane, g.k), T, (RW)eq, D.reach, l, end, U, Lf);
@@ -322,7 +191,7 @@ __device__ __forceinline__ int diag_align(const Segment &g, const DiagSpan &s, c
 
 // One warp tile; `next`: the tile after it (its offsets arrive while this
 // one is aligned, its bytes go to L2 while this one's strings are written).
-template <bool ROWS>
+template <class F>
 __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &now, int next,
                                          TileAhead &ahead, int lane, uint8_t *slice_p, Sm gaps) {
   const Segment &g = a.segs[now.seg];
@@ -341,7 +210,7 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
                           g.first_of_call && t0 + lane == 0, lane < count, l)
                ? 0
                : 1;
-  const DiagLayout D = diag_layout(g.max_m, k, ROWS);
+  const DiagLayout D = diag_layout(g.max_m, k, F::ROWS, F::CELL);
   const Sm slice = sm_at(slice_p);
   uint32_t odd = 0;
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -371,7 +240,7 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
   auto finish = [&]() {
     if (!more || !fits_next) return;
     const Segment &h = a.segs[ahead.seg];
-    const DiagLayout N = diag_layout(h.max_m, h.k, ROWS);
+    const DiagLayout N = diag_layout(h.max_m, h.k, F::ROWS, F::CELL);
     stage_tile(h, sn, slice, slice + N.src_r, lane);
   };
   if (!fits) {  // offsets no regular call can have: report, do not stage
@@ -385,7 +254,7 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
   __syncwarp();
   WalkEnd end;
   const bool any_odd = __any_sync(0xffffffffu, odd != 0);
-  st |= diag_align<ROWS>(g, s, D, any_odd, lane, slice, l, end, U, Lf);
+  st |= diag_align<F>(g, s, D, any_odd, lane, slice, l, end, U, Lf);
   __syncwarp();
   prefetch();
   if (lane < count) g.scores[t0 + lane] = l.score;
@@ -435,7 +304,7 @@ constexpr int kDiagWarpsPerSm = 4 * kDiagCtas;
 
 // Persistent warps: the first tile of a warp is its own number, later ones
 // come from the launch's counter (none: the grid has a warp for every tile).
-template <bool ROWS>
+template <class F>
 __global__ void __launch_bounds__(128, kDiagCtas)
     saru_diag_kernel(const __grid_constant__ KernelArgs a) {
   extern __shared__ uint4 smem_v[];
@@ -451,7 +320,7 @@ __global__ void __launch_bounds__(128, kDiagCtas)
   tile_ahead(a, first, lane, now);
   {
     const Segment &g = a.segs[now.seg];
-    const DiagLayout D = diag_layout(g.max_m, g.k, ROWS);
+    const DiagLayout D = diag_layout(g.max_m, g.k, F::ROWS, F::CELL);
     DiagSpan s;
     const Sm raw = sm_at(slice);
     if (tile_span(a, now, 32, s)) stage_tile(g, s, raw, raw + D.src_r, lane);
@@ -463,7 +332,7 @@ __global__ void __launch_bounds__(128, kDiagCtas)
       next = __shfl_sync(0xffffffffu, next, 0);
     }
     TileAhead ahead;
-    int status = diag_tile<ROWS>(a, now, next, ahead, lane, slice, sm_at(gaps));
+    int status = diag_tile<F>(a, now, next, ahead, lane, slice, sm_at(gaps));
     status = __reduce_or_sync(0xffffffffu, status);
     if (status && lane == 0)
       atomicOr(a.segs[now.seg].status,
@@ -668,6 +537,9 @@ __global__ void saru_full_trace_kernel(FullArgs a) {
 
 constexpr long kMaxCtaSmem = 227 * 1024;  // opt-in shared memory per block on sm_100
 
+// The scratch a caller provides is sized as it always was, by the banded form
+// (band_tile.cuh): per lane of a persistent grid, the decision planes of its
+// read length.  The diagonal kernel uses the tile counter at its start.
 BandLayout band_layout(int max_m, int k, int warps_req, bool wide) {
   const SliceLayout S = slice_layout(max_m, k, wide);
   BandLayout L;
@@ -696,11 +568,14 @@ cudaError_t allow_smem() {
   std::lock_guard<std::mutex> lk(g_attr_mu);
   if ((g_attr_done >> dev) & 1u) return cudaSuccess;
   const int attr = cudaFuncAttributeMaxDynamicSharedMemorySize, most = (int)kMaxCtaSmem;
-  e = cudaFuncSetAttribute(saru_band_kernel, (cudaFuncAttribute)attr, most);
+  e = cudaFuncSetAttribute(saru_diag_kernel<DiagForm<true, 1>>, (cudaFuncAttribute)attr,
+                             most - 64);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(saru_diag_kernel<true>, (cudaFuncAttribute)attr, most - 64);
+    e = cudaFuncSetAttribute(saru_diag_kernel<DiagForm<false, 1>>, (cudaFuncAttribute)attr,
+                             most - 64);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(saru_diag_kernel<false>, (cudaFuncAttribute)attr, most - 64);
+    e = cudaFuncSetAttribute(saru_diag_kernel<DiagForm<false, 2>>, (cudaFuncAttribute)attr,
+                             most - 64);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(saru_full_fill_rows_kernel<true>, (cudaFuncAttribute)attr, most);
   if (e == cudaSuccess)
@@ -710,16 +585,13 @@ cudaError_t allow_smem() {
 }
 }  // namespace
 
-// The diagonal kernel takes every launch whose reads fit its byte columns;
-// the banded one the longer reads.
-bool diag_launch(int max_m) { return max_m <= kDiagMaxM; }
-
 // The largest slice a launch's segments need (a slice does not grow with
 // the read length and k in every case, so it is not the longest read's).
 long diag_slice(const KernelArgs &a, bool rows) {
+  const int cell = a.max_m <= kByteColumns ? 1 : 2;
   long most = 0;
   for (int i = 0; i < a.nseg; ++i) {
-    const long s = diag_layout(a.segs[i].max_m, a.segs[i].k, rows).slice;
+    const long s = diag_layout(a.segs[i].max_m, a.segs[i].k, rows, cell).slice;
     if (s > most) most = s;
   }
   return most;
@@ -727,9 +599,9 @@ long diag_slice(const KernelArgs &a, bool rows) {
 
 // Whether a launch looks its mismatches up in rows: one word has a bit per
 // diagonal -k .. 5k/2 up to k = 9, a row's columns past m must fit a byte, and
-// the slice must leave room for enough warps.  Rows take 68 us where planes
-// take 88 for 176k candidates of 100 bp at k = 5 (14 KB a slice against 16),
-// 70 against 50 for 41k of 133 bp at k = 8 (29 KB against 21).
+// the slice must leave room for enough warps.  Rows take 65 us where planes
+// take 73 for 176k candidates of 100 bp at k = 5 (13.6 KB a slice either way),
+// 66 against 47 for 41k of 133 bp at k = 8 (27 KB against 17).
 constexpr long kRowsSlice = 20 * 1024;
 bool diag_rows(const KernelArgs &a) {
   return a.max_k <= 9 && a.max_m <= 200 && diag_slice(a, true) <= kRowsSlice;
@@ -779,24 +651,11 @@ cudaError_t launch_diag_kernel(KernelArgs &a, int sms, int smem_per_sm, int ctas
     if (e != cudaSuccess) return e;
   }
   const size_t smem = (size_t)(a.warp_smem * warps);
-  if (rows) saru_diag_kernel<true><<<(unsigned)a.grid, 32 * warps, smem, s>>>(a);
-  else saru_diag_kernel<false><<<(unsigned)a.grid, 32 * warps, smem, s>>>(a);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_band_kernel(KernelArgs &a, cudaStream_t s) {
-  const BandLayout L = band_layout(a.max_m, a.max_k, a.warps_req, a.wide_any != 0);
-  if (L.warps < 1 || a.nseg < 1 || a.nseg > kMaxSegs) return cudaErrorInvalidValue;
-  // allow the largest slice once per device; each launch asks for its own
-  // size (a per-launch attribute would race between concurrent callers)
-  cudaError_t e = allow_smem();
-  if (e != cudaSuccess) return e;
-  a.rs_bytes = L.rs_bytes;
-  a.ws_bytes = L.ws_bytes;
-  a.warp_smem = L.warp_smem;
-  e = cudaMemsetAsync(a.counter, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
-  saru_band_kernel<<<(unsigned)a.grid, 32 * L.warps, L.cta_smem, s>>>(a);
+  const unsigned grid = (unsigned)a.grid, threads = 32 * (unsigned)warps;
+  if (rows) saru_diag_kernel<DiagForm<true, 1>><<<grid, threads, smem, s>>>(a);
+  else if (a.max_m <= kByteColumns)
+    saru_diag_kernel<DiagForm<false, 1>><<<grid, threads, smem, s>>>(a);
+  else saru_diag_kernel<DiagForm<false, 2>><<<grid, threads, smem, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -33,7 +33,7 @@ struct Segment {
   long n;           // candidates t0 .. n - 1 of the call's arrays are this segment's
   long t0;          // (t0 > 0, a multiple of 32: a later slice of a call)
   long tile_begin;  // first 32-candidate tile of this segment in the launch
-  int k, max_m, first_of_call, wide;
+  int k, max_m, first_of_call;
 };
 
 constexpr int kMaxSegs = 192;         // segments per launch (kernel parameter space)
@@ -43,21 +43,19 @@ struct KernelArgs {
   Segment segs[kMaxSegs];  // by value in the parameter space
   int nseg;
   long total_tiles;
-  int *counter;  // zeroed before the launch: next tile to take
-  void *planes;  // decision planes: plane_units(max_m, wide_any) x lanes units (band_tile.cuh)
+  int *counter;  // next tile to take, zeroed before the launch (nullptr: a warp for every tile)
   long grid;
-  int max_m, max_k, wide_any;
+  int max_m, max_k;
   int warps_req;                       // requested warps per CTA (0: as many as fit)
-  long rs_bytes, ws_bytes, warp_smem;  // shared-memory slice layout (set by the launcher)
+  long warp_smem;                      // a warp's shared-memory slice (set by the launcher)
 };
 
-// Launch shape of the banded kernel for one (read length, k) class; 0 keeps
-// the default (as many warps per CTA and CTAs per SM as fit; 32-bit band
-// words when k <= 7).
+// Launch shape of the alignment kernel for one (read length, k) class; 0
+// keeps the default (as many warps per CTA and CTAs per SM as fit).
 struct Tuning {
   int warps = 0;        // warps per CTA, 1..4
   int ctas_per_sm = 0;  // cap on resident CTAs per SM
-  int word_bits = 0;    // 64: 64-bit band words even when k <= 7
+  int word_bits = 0;    // 64: scratch sized for 64-bit band words even when k <= 7
 };
 
 struct BandLayout {
@@ -111,8 +109,6 @@ BandLayout band_layout(int max_m, int k, int warps_req = 0, bool wide = true);
 long band_grid(int sms, long n, const BandLayout &L, int smem_per_sm, int ctas_cap = 0);
 size_t band_scratch_bytes(long grid, int max_m, int k, bool wide,
                           int warps_req = 0);  // counter + planes
-cudaError_t launch_band_kernel(KernelArgs &a, cudaStream_t s);
-bool diag_launch(int max_m);  // whether a launch's reads go to the diagonal kernel
 cudaError_t launch_diag_kernel(KernelArgs &a, int sms, int smem_per_sm, int ctas_cap,
                                cudaStream_t s);
 cudaError_t launch_full_kernels(const FullArgs &a, cudaStream_t s);

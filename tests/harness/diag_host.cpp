@@ -17,8 +17,8 @@ static Quad load16(const uint8_t *p) {
   return q;
 }
 
-template <typename RW, class X>
-static int lane(const X &P, const DiagTable &T, RW eq, int reach, DiagLane &ls, WalkEnd &end,
+template <typename RW, class X, class Table>
+static int lane(const X &P, const Table &T, RW eq, int reach, DiagLane &ls, WalkEnd &end,
                 const GapMask &U, const GapMask &Lf) {
   const DiagExit x = lane_levels<RW>(ls.c, P, T, eq, reach);
   ls.score = x.score;
@@ -29,9 +29,10 @@ static int lane(const X &P, const DiagTable &T, RW eq, int reach, DiagLane &ls, 
   return 4;
 }
 
-template <bool ROWS, bool ODD>
+template <class F, bool ODD>
 static int align(const TileArgs &a, const DiagSpan &s, const DiagLayout &D, Sm slice,
                  DiagLane *ls, WalkEnd *end, const GapMask *U, const GapMask *Lf) {
+  constexpr bool ROWS = F::ROWS;
   using RW = typename DiagWord<ROWS>::type;
   int st = 0;
   RW eq[32] = {};
@@ -66,7 +67,7 @@ static int align(const TileArgs &a, const DiagSpan &s, const DiagLayout &D, Sm s
   for (int i = 0; i < 32; ++i) {
     end[i] = WalkEnd{0, 0, 0, false};
     if (!ls[i].ok) continue;
-    const DiagTable T(table, i, a.k);
+    const DiagTable<F::CELL> T(table, i, a.k);
     const MismatchRows M(slice, D, i, a.k);
     const Planes<ODD> P(slice, D, i, a.k);
     st |= ROWS ? lane<RW>(M, T, eq[i], D.reach, ls[i], end[i], U[i], Lf[i])
@@ -76,9 +77,9 @@ static int align(const TileArgs &a, const DiagSpan &s, const DiagLayout &D, Sm s
   return st;
 }
 
-template <bool ROWS>
+template <class F>
 static int run(const TileArgs &a) {
-  const DiagLayout D = diag_layout(a.max_m, a.k, ROWS);
+  const DiagLayout D = diag_layout(a.max_m, a.k, F::ROWS, F::CELL);
   uint8_t *slice_p = (uint8_t *)aligned_alloc(16, (size_t)D.slice);
   memset(slice_p, 0xA5, (size_t)D.slice);
   const Sm slice = sm_at(slice_p);
@@ -127,8 +128,8 @@ static int run(const TileArgs &a) {
       U[lane] = GapMask{masks};
       Lf[lane] = GapMask{masks + D.mwords * 128};
     }
-    status |= odd ? align<ROWS, true>(a, s, D, slice, ls, end, U, Lf)
-                  : align<ROWS, false>(a, s, D, slice, ls, end, U, Lf);
+    status |= odd ? align<F, true>(a, s, D, slice, ls, end, U, Lf)
+                  : align<F, false>(a, s, D, slice, ls, end, U, Lf);
     for (int lane = 0; lane < 32; ++lane) {
       const long t = t0 + lane;
       if (t >= a.n) continue;
@@ -175,5 +176,6 @@ extern "C" int diag_align_batch(const uint8_t *genome, const uint8_t *reads, con
                                 uint8_t *ga, uint8_t *records, long rec_bytes) {
   TileArgs a{genome, reads, goff, roff, dirs, n, k, max_m, first_of_call, scores, ra, ga,
              nullptr, 0, 0, 0, 0, records, rec_bytes, t0};
-  return rows ? run<true>(a) : run<false>(a);
+  if (rows) return run<DiagForm<true, 1>>(a);
+  return max_m <= kByteColumns ? run<DiagForm<false, 1>>(a) : run<DiagForm<false, 2>>(a);
 }

@@ -18,10 +18,10 @@ ROOT = Path(__file__).resolve().parents[1]
 SRC = ROOT / "tests" / "harness" / "diag_host.cpp"
 SO = ROOT / "tests" / "_build" / "libdiag_host_asan.so"
 
-# read length, k: edges of the 32-column words, of the byte table (255) and
+# read length, k: edges of the 32-column words, of the byte table (255 / 256) and
 # of the 32-bit diagonal word (k = 9 / 10), m = 3k + 1, the smallest reads
 SHAPES = [(36, 2), (100, 5), (31, 3), (32, 1), (33, 4), (64, 7), (95, 9), (128, 10), (150, 9),
-          (250, 15), (255, 12), (46, 15), (2, 0), (8, 1), (40, 13), (16, 5)]
+          (250, 15), (255, 12), (46, 15), (2, 0), (8, 1), (40, 13), (16, 5), (256, 12), (300, 9), (512, 15)]
 
 
 def exact(a: np.ndarray, off: int) -> np.ndarray:

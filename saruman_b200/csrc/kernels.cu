@@ -303,7 +303,7 @@ constexpr int kDiagCtas = 4;
 constexpr int kDiagWarpsPerSm = 4 * kDiagCtas;
 
 // Persistent warps: the first tile of a warp is its own number, later ones
-// come from the launch's counter (none: the grid has a warp for every tile).
+// come from the launch's counter (none: in turn).
 template <class F>
 __global__ void __launch_bounds__(128, kDiagCtas)
     saru_diag_kernel(const __grid_constant__ KernelArgs a) {
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(128, kDiagCtas)
     if (tile_span(a, now, 32, s)) stage_tile(g, s, raw, raw + D.src_r, lane);
   }
   while (now.tile < a.total_tiles) {
-    int next = (int)a.total_tiles;
+    int next = now.tile + (int)gridDim.x * warps;
     if (a.counter) {
       if (lane == 0) next = (int)gridDim.x * warps + atomicAdd(a.counter, 1);
       next = __shfl_sync(0xffffffffu, next, 0);
@@ -630,6 +630,12 @@ int diag_warps(long slice, int warps_req, int smem_per_sm) {
   return warps;
 }
 
+// Launches of up to this many tiles a warp take them in turn (no counter to
+// clear and to wait for): 176k candidates of 100 bp (2.3 tiles a warp) 65.4 ->
+// 61.6 us, mixed lengths 168 -> 161; at 12 tiles a warp the counter is 1 %
+// faster.
+constexpr int kStaticRounds = 4;
+
 cudaError_t launch_diag_kernel(KernelArgs &a, int sms, int smem_per_sm, int ctas_cap,
                                cudaStream_t s) {
   if (a.nseg < 1 || a.nseg > kMaxSegs) return cudaErrorInvalidValue;
@@ -644,8 +650,8 @@ cudaError_t launch_diag_kernel(KernelArgs &a, int sms, int smem_per_sm, int ctas
   if (ctas_cap >= 1 && per_sm > ctas_cap) per_sm = ctas_cap;
   const long ctas = (a.total_tiles + warps - 1) / warps;
   a.grid = ctas < sms * per_sm ? ctas : sms * per_sm;
-  if (a.total_tiles <= a.grid * warps) {
-    a.counter = nullptr;  // a warp for every tile
+  if (a.total_tiles <= kStaticRounds * a.grid * warps) {
+    a.counter = nullptr;
   } else {
     e = cudaMemsetAsync(a.counter, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;

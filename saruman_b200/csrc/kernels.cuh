@@ -43,7 +43,7 @@ struct KernelArgs {
   Segment segs[kMaxSegs];  // by value in the parameter space
   int nseg;
   long total_tiles;
-  int *counter;  // next tile to take, zeroed before the launch (nullptr: a warp for every tile)
+  int *counter;  // next tile to take, zeroed before the launch (nullptr: tiles in turn)
   long grid;
   int max_m, max_k;
   int warps_req;                       // requested warps per CTA (0: as many as fit)

@@ -213,8 +213,8 @@ def measured_peaks() -> dict:
 
 def profile_traffic() -> dict | None:
     """DRAM bytes per candidate of the banded kernel from the committed ncu
-    summary (profiles/band_kernel_c2.json), if present."""
-    p = ROOT / "profiles" / "band_kernel_c2.json"
+    summary (profiles/diag_kernel_c2.json), if present."""
+    p = ROOT / "profiles" / "diag_kernel_c2.json"
     if p.exists():
         try:
             return json.loads(p.read_text())
@@ -963,7 +963,7 @@ def run_aligner(args, cfg: dict, rank: int, world: int, local: int) -> None:
         "peak": int_peak / 1e12 if int_peak and int_peak > 0 else None,
         "unit": "Tops/s", "frac": (achieved_ops / int_peak) if int_peak and int_peak > 0 else None,
         "traffic": traffic,
-        "traffic_source": "profiles/band_kernel_c2.json (ncu dram bytes per candidate, small case, "
+        "traffic_source": "profiles/diag_kernel_c2.json (ncu dram bytes per candidate, small case, "
                           "scaled by candidates)" if traffic else None,
         "peak_source": "measured live by saru_int32_issue_probe on this GPU",
         "ops_per_candidate_definition": "band cells x 6 (m*(2k+1) or m*(4k+1) cells)",

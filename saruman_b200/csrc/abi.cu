@@ -1137,8 +1137,8 @@ int saru_align_device(const saru_batch *batch, saru_result *result, void *scratc
 
 // ---------------------------------------------------------------------------
 // Entry point without any device allocation.  Its scratch (the banded
-// kernel's decision planes) is this file-scope device array, present on
-// every GPU that loads the library for the life of the process.
+// kernel's tile counter) is at the start of this file-scope device array,
+// present on every GPU that loads the library for the life of the process.
 // ---------------------------------------------------------------------------
 namespace {
 

@@ -1,4 +1,8 @@
-// band_tile.cuh -- one warp tile of the banded kernel, as phases.
+// band_tile.cuh -- one warp tile of a bit-parallel band, as phases.
+//
+// The device kernel (diag_tile.cuh) shares its staging, its copy-out and its
+// bit helpers; the band's own phases run in the host tests, and its sizes are
+// what callers' scratch is still checked against.
 //
 // A warp tile is 32 consecutive candidates, one per lane.  Their reads,
 // windows and output slots are three contiguous byte ranges, so the warp

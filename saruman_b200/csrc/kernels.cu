@@ -296,8 +296,8 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
   return st;
 }
 
-// 16 warps an SM: 104 registers a thread leave room for more, but the slices
-// do not (14.2 KB at 100 bp, k = 5).  Held to 3 or 5 CTAs of 4 warps: 332 or
+// 16 warps an SM: registers (106 a thread) and slices (13.8 KB at 100 bp, k = 5)
+// both end there.  Held to 3 or 5 CTAs of 4 warps: 332 or
 // 294 us against 291 for 930k candidates of 100 bp.
 constexpr int kDiagCtas = 4;
 constexpr int kDiagWarpsPerSm = 4 * kDiagCtas;

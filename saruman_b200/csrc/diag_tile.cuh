@@ -19,6 +19,7 @@
 // The phases are separated by warp barriers in the kernel; written as
 // functions of the lane so a host harness can run them lane by lane.
 #pragma once
+#include <assert.h>
 #include <stdint.h>
 
 #include "band_tile.cuh"
@@ -29,11 +30,13 @@ namespace saru {
 // longer ones.
 constexpr int kByteColumns = 255;
 
-// The forms a launch runs in: `rows` or planes (DiagLayout), bytes a cell.
-template <bool ROWS_, int CELL_>
+// The forms a launch runs in: `rows` or planes (DiagLayout), bytes a cell, and
+// whether rows cut columns at m (columns_cross).
+template <bool ROWS_, int CELL_, bool CUT_ = false>
 struct DiagForm {
   static constexpr bool ROWS = ROWS_;
   static constexpr int CELL = CELL_;
+  static constexpr bool CUT = CUT_;
 };
 
 struct alignas(16) Quad {
@@ -160,7 +163,10 @@ inline int sm_ld8(Sm p) { return *p.a; }
 inline int sm_ld16(Sm p) { return *reinterpret_cast<uint16_t *>(p.a); }
 inline uint32_t sm_ld32(Sm p) { return *reinterpret_cast<uint32_t *>(p.a); }
 inline Quad sm_ld128(Sm p) { return *reinterpret_cast<Quad *>(p.a); }
-inline void sm_st8(Sm p, int v) { *p.a = (uint8_t)v; }
+inline void sm_st8(Sm p, int v) {
+  assert(v >= 0 && v <= 255);  // a table cell of one byte holds the column
+  *p.a = (uint8_t)v;
+}
 inline void sm_st16(Sm p, uint32_t v) { *reinterpret_cast<uint16_t *>(p.a) = (uint16_t)v; }
 inline void sm_st32(Sm p, uint32_t v) { *reinterpret_cast<uint32_t *>(p.a) = v; }
 inline void sm_st128(Sm p, Quad q) { *reinterpret_cast<Quad *>(p.a) = q; }
@@ -243,6 +249,13 @@ SARU_HD DiagLayout diag_layout(int max_m, int k, bool rows, int cell) {
   D.slice = front + D.masks_bytes;
   return D;
 }
+
+// On a diagonal that has reached column m a level's start goes on one column
+// past the level before's, so level e looks at column m + e.  Whether such a
+// column leaves its diagonal's row (whose words end with the one of column m +
+// 1) for the next diagonal's first columns: then columns have to be cut at m.
+// Reads shorter than max_m do not cross if max_m does not.
+SARU_HD bool columns_cross(int max_m, int k) { return ((max_m + k) >> 5) > ((max_m + 1) >> 5); }
 
 // ---------------------------------------------------------------------------
 // planes
@@ -407,14 +420,17 @@ SARU_HD bool read_extras(const StreamWords &s, int words, int len, const uint8_t
 }
 
 // Mismatch bits of a lane by diagonal: word w of diagonal d holds columns
-// 32w .. (column j, 1-based, is position j; position 0 is padding).
-struct MismatchRows {
+// 32w .. (column j, 1-based, is position j; position 0 is padding).  CUT: see
+// columns_cross.
+template <bool CUT>
+struct RowsOf {
   Sm zero;     // diagonal 0
   int stride;  // bytes from a diagonal to the next
   int k;
   typedef Sm Row;
   static constexpr bool kStops = true;  // columns from m on count as mismatches
-  SARU_HD MismatchRows(Sm slice, const DiagLayout &D, int lane, int k_)
+  static constexpr bool kCut = CUT;
+  SARU_HD RowsOf(Sm slice, const DiagLayout &D, int lane, int k_)
       : zero(slice + (k_ * D.nr * 128 + lane * 4)), stride(D.nr * 128), k(k_) {}
   SARU_HD Row row(int d) const { return zero + d * stride; }
   SARU_HD Row next(Row r) const { return r + stride; }
@@ -426,6 +442,9 @@ struct MismatchRows {
   }
 };
 
+using MismatchRows = RowsOf<true>;
+using MismatchRowsUncut = RowsOf<false>;
+
 // Columns m and later of word w.
 SARU_HD uint32_t past_columns(int m, int w) {
   const int c = 32 * (w + 1) - m;
@@ -433,9 +452,9 @@ SARU_HD uint32_t past_columns(int m, int w) {
 }
 
 // Diagonals whose last column matches: bit reach - d.
-template <bool ODD>
+template <bool ODD, class Rows>
 SARU_HD uint32_t row_matches(const StreamWords &R, const StreamWords &W, int m, int reach,
-                             const MismatchRows &M) {
+                             const Rows &M) {
   if (!ODD) {  // the last read position against window rows m - k ..
     const uint32_t a = 0u - (R.from(R.s0, m) >> 31), b = 0u - (R.from(R.s1, m) >> 31);
     const uint32_t ne = (a ^ W.from(W.s0, m - M.k)) | (b ^ W.from(W.s1, m - M.k));
@@ -452,10 +471,10 @@ SARU_HD uint32_t row_matches(const StreamWords &R, const StreamWords &W, int m, 
 // word: two funnel shifts of the window (its words taken from row -k on, so
 // diagonal d is a shift by d + k < 32), two three-input logic operations, a
 // store.
-template <bool ODD>
+template <bool ODD, class Rows>
 SARU_HD uint32_t lane_rows(const StreamWords &R, const StreamWords &W, const Cand &c,
                            const uint8_t *read, const uint8_t *win, const Extras &x,
-                           const DiagLayout &D, const MismatchRows &M) {
+                           const DiagLayout &D, const Rows &M) {
   const int m = c.m, L = c.L, k = M.k;
   Bits3 here = plane_words<ODD>(W, -k, L, win, x);
   for (int w = 0; w < D.nr; ++w) {
@@ -498,6 +517,7 @@ struct Planes {
   int k;
   typedef int Row;
   static constexpr bool kStops = false;
+  static constexpr bool kCut = true;  // entries end with the word of column m + 1
   SARU_HD Planes(Sm slice, const DiagLayout &D, int lane, int k_)
       : rd(slice + lane * 16), wn(slice + (lane * 16 + (D.nr + 1) * 512)), k(k_) {}
   SARU_HD Bits3 bits(Sm seq, int pos) const {
@@ -596,7 +616,7 @@ struct DiagExit {
   int v;      // value of the next cell (in column m for OP_UP)
 };
 
-// Levels 0 .. k of one lane.  X: its mismatches (MismatchRows or Planes);
+// Levels 0 .. k of one lane.  X: its mismatches (RowsOf or Planes);
 // eq: the diagonals whose last column matches (RW: bit reach - d).
 //
 // Bound by instruction issue: about 17 instructions a cell on rows (the
@@ -639,7 +659,7 @@ SARU_HD DiagExit lane_levels(const Cand &c, const X &P, const Table &T, RW eq, i
     };
     // (level k is not stored: the walk asks for lower values only)
     auto keep = [&](Sm to, int s) {
-      if (!X::kStops) s = s < m ? s : m;
+      if (X::kCut) s = s < m ? s : m;
       short_of = push_sign(short_of, s - m);
       if (e < k) Table::put(to, s);
     };

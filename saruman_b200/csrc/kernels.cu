@@ -115,7 +115,7 @@ __device__ __forceinline__ void stage_tile(const Segment &g, const DiagSpan &s, 
 
 // The lanes' compare parts from the tile's bit streams; the alphabet status
 // bit.  eq: row_matches (rows form).
-template <bool ROWS, bool ODD>
+template <class F, bool ODD>
 __device__ __forceinline__ int diag_compare(const Segment &g, const DiagSpan &s,
                                             const DiagLayout &D, int lane, Sm slice, DiagLane &l,
                                             uint32_t &eq) {
@@ -135,8 +135,8 @@ __device__ __forceinline__ int diag_compare(const Segment &g, const DiagSpan &s,
     st = 2;  // alphabet
     l.ok = false;
   }
-  if (ROWS) {
-    if (l.ok) eq = lane_rows<ODD>(R, W, l.c, read, win, x, D, MismatchRows(slice, D, lane, g.k));
+  if (F::ROWS) {
+    if (l.ok) eq = lane_rows<ODD>(R, W, l.c, read, win, x, D, RowsOf<F::CUT>(slice, D, lane, g.k));
   } else {
     const Planes<ODD> P(slice, D, lane, g.k);
     lane_planes<ODD>(R, D.nr, l.ok ? l.c.m : 0, read, x, false, P.rd);
@@ -167,8 +167,8 @@ __device__ __forceinline__ int diag_align(const Segment &g, const DiagSpan &s, c
   constexpr bool ROWS = F::ROWS;
   using RW = typename DiagWord<ROWS>::type;
   uint32_t eq = 0;
-  int st = odd ? diag_compare<ROWS, true>(g, s, D, lane, slice, l, eq)
-               : diag_compare<ROWS, false>(g, s, D, lane, slice, l, eq);
+  int st = odd ? diag_compare<F, true>(g, s, D, lane, slice, l, eq)
+               : diag_compare<F, false>(g, s, D, lane, slice, l, eq);
   __syncwarp();
   const Sm table = slice + D.compare_bytes;
   // table and gap masks (adjacent) start from zero
@@ -179,7 +179,8 @@ __device__ __forceinline__ int diag_align(const Segment &g, const DiagSpan &s, c
   const DiagTable<F::CELL> T(table, lane, g.k);
   if (!l.ok) return st;
   if (ROWS)
-    return st | diag_lane<RW>(MismatchRows(slice, D, lane, g.k), T, (RW)eq, D.reach, l, end, U, Lf);
+    return st | diag_lane<RW>(RowsOf<F::CUT>(slice, D, lane, g.k), T, (RW)eq, D.reach, l, end, U,
+                              Lf);
   const int m = l.c.m;
   if (odd) {
     const Planes<true> P(slice, D, lane, g.k);
@@ -586,6 +587,9 @@ cudaError_t allow_smem() {
   e = cudaFuncSetAttribute(saru_diag_kernel<DiagForm<true, 1>>, (cudaFuncAttribute)attr,
                              most - 64);
   if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(saru_diag_kernel<DiagForm<true, 1, true>>, (cudaFuncAttribute)attr,
+                             most - 64);
+  if (e == cudaSuccess)
     e = cudaFuncSetAttribute(saru_diag_kernel<DiagForm<false, 1>>, (cudaFuncAttribute)attr,
                              most - 64);
   if (e == cudaSuccess)
@@ -613,13 +617,26 @@ long diag_slice(const KernelArgs &a, bool rows) {
 }
 
 // Whether a launch looks its mismatches up in rows: one word has a bit per
-// diagonal -k .. 5k/2 up to k = 9, a row's columns past m must fit a byte, and
-// the slice must leave room for enough warps.  Rows take 65 us where planes
-// take 73 for 176k candidates of 100 bp at k = 5 (13.6 KB a slice either way),
-// 66 against 47 for 41k of 133 bp at k = 8 (27 KB against 17).
+// diagonal -k .. 5k/2 up to k = 9, the columns that a row is looked up at (up to
+// m + k) must fit a byte, and the slice must leave room for enough warps.  Rows take 65 us where planes take 73 for 176k candidates of
+// 100 bp at k = 5 (slices of 13.8 and 12.0 KB), 66 against 47 for 41k of 133 bp
+// at k = 8 (27.9 KB against 15.9).
 constexpr long kRowsSlice = 20 * 1024;
+constexpr int kRowsMaxK = 9, kRowsMaxM = 200;
+static_assert(kRowsMaxM + kRowsMaxK <= kByteColumns, "a table cell is a byte");
 bool diag_rows(const KernelArgs &a) {
-  return a.max_k <= 9 && a.max_m <= 200 && diag_slice(a, true) <= kRowsSlice;
+  return a.max_k <= kRowsMaxK && a.max_m <= kRowsMaxM && diag_slice(a, true) <= kRowsSlice;
+}
+
+// Whether a launch's rows cut columns at m.  An instruction a cell, so only
+// launches with a read length that needs it do: cut everywhere, 176k
+// candidates of 100 bp take 62.7 us instead of 62.2, 930k 281.9 instead of 279.9.
+// (Rows long enough for column m + k instead: 120k of 94 bp at k = 6 67.6 us
+// against 55.3 cut, of 158 bp at k = 6 91.6 against 84.0.)
+bool diag_cut(const KernelArgs &a) {
+  for (int i = 0; i < a.nseg; ++i)
+    if (columns_cross(a.segs[i].max_m, a.segs[i].k)) return true;
+  return false;
 }
 
 // CTAs of w warps (shared memory w slices) an SM holds.
@@ -673,7 +690,8 @@ cudaError_t launch_diag_kernel(KernelArgs &a, int sms, int smem_per_sm, int ctas
   }
   const size_t smem = (size_t)(a.warp_smem * warps);
   const unsigned grid = (unsigned)a.grid, threads = 32 * (unsigned)warps;
-  if (rows) saru_diag_kernel<DiagForm<true, 1>><<<grid, threads, smem, s>>>(a);
+  if (rows && diag_cut(a)) saru_diag_kernel<DiagForm<true, 1, true>><<<grid, threads, smem, s>>>(a);
+  else if (rows) saru_diag_kernel<DiagForm<true, 1>><<<grid, threads, smem, s>>>(a);
   else if (a.max_m <= kByteColumns)
     saru_diag_kernel<DiagForm<false, 1>><<<grid, threads, smem, s>>>(a);
   else saru_diag_kernel<DiagForm<false, 2>><<<grid, threads, smem, s>>>(a);

@@ -266,6 +266,9 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
       rec[0] = (uint32_t)end.n | (end.bad ? 0x10000u : 0u);
       record_words(end.n, nwords, U, Lf, [&](int w, uint32_t v) { rec[w] = v; });
     }
+    // the next tile may be another segment's, whose staged bytes reach over
+    // this one's gap masks
+    __syncwarp();
     finish();
     return st;
   }

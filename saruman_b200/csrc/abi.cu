@@ -211,32 +211,67 @@ struct PlanPart {
   bool uniform = true, regular = true, start_gap = false;
 };
 
-// (in locals, stored once at the end: the parts of the threads share cache
-// lines)
-void plan_range(const saru_batch *b, int lo, int hi, PlanPart *out) {
-  const int k = b->k;
+// One candidate after the other; false at an invalid one.
+bool plan_each(const saru_batch *b, int lo, int hi, PlanPart &p) {
   const int32_t *go = b->genome_offsets, *ro = b->read_offsets;
-  const int8_t *dirs = b->dirs;
-  int64_t prev_g = lo ? go[lo - 1] : 0;
-  int64_t prev_r = lo ? ro[lo - 1] : 0;
-  PlanPart p;
   for (int t = lo; t < hi; ++t) {
-    const int64_t L = (int64_t)go[t] - prev_g;
-    const int64_t m = (int64_t)ro[t] - prev_r;
+    const int64_t L = (int64_t)go[t] - (t ? go[t - 1] : 0);
+    const int64_t m = (int64_t)ro[t] - (t ? ro[t - 1] : 0);
     if (L <= 0 || m <= 0 || L > 32000 || m > 32000) {
       p.bad = t;
-      break;
+      return false;
     }
-    prev_g = go[t];
-    prev_r = ro[t];
     if (p.m_first < 0) p.m_first = (int)m;
     p.uniform &= m == p.m_first;
     if (m > p.max_m) p.max_m = (int)m;
     int so, eo;
-    saru::flank_of(dirs[t], k, so, eo);
+    saru::flank_of(b->dirs[t], b->k, so, eo);
     p.start_gap |= so != 0;
     p.regular &= L == m + so + eo;
     p.cells += (m + 1) * (L + 1);
+  }
+  return true;
+}
+
+// Whether candidates [t0, t1) (t0 > 0) all have reads of m bases and windows of
+// m + so + eo; *flags: their flags, ORed.  A few operations on 32 bits a
+// candidate, eight candidates at once: 0.4 ns where plan_each takes 2.8.
+__attribute__((target_clones("avx2", "default"))) bool plan_regular(
+    const int32_t *go, const int32_t *ro, const int8_t *dirs, int t0, int t1, uint32_t m,
+    uint32_t k, uint32_t *flags) {
+  uint32_t other = 0, all = 0;
+  int32_t sign = go[t0 - 1] | ro[t0 - 1];
+  for (int t = t0; t < t1; ++t) {
+    const uint32_t d = (uint32_t)(int32_t)dirs[t];
+    const uint32_t so = (0u - ((d >> 1) & 1u)) & k, eo = (0u - (d & 1u)) & k;  // flank_of
+    other |= ((uint32_t)ro[t] - (uint32_t)ro[t - 1]) ^ m;
+    other |= ((uint32_t)go[t] - (uint32_t)go[t - 1]) ^ (m + so + eo);
+    all |= d;
+    sign |= go[t] | ro[t];  // (offsets that are not negative: differences are exact)
+  }
+  *flags = all;
+  return other == 0 && sign >= 0 && all <= 7u;
+}
+
+// Blocks of regular candidates at once, others one by one (in locals, stored
+// once at the end: the parts of the threads share cache lines).
+void plan_range(const saru_batch *b, int lo, int hi, PlanPart *out) {
+  constexpr int kBlock = 1024;
+  const int32_t *go = b->genome_offsets, *ro = b->read_offsets;
+  const uint32_t k = (uint32_t)b->k;
+  PlanPart p;
+  bool ok = lo >= hi || plan_each(b, lo, lo + 1, p);
+  for (int t0 = lo + 1; ok && t0 < hi; t0 += kBlock) {
+    const int t1 = std::min(hi, t0 + kBlock);
+    const uint32_t m = (uint32_t)p.m_first;
+    uint32_t flags = 0;
+    if (k > 15u || m + 2 * k > 32000u ||
+        !plan_regular(go, ro, b->dirs, t0, t1, m, k, &flags)) {
+      ok = plan_each(b, t0, t1, p);
+      continue;
+    }
+    p.start_gap |= k > 0 && (flags & 2u);
+    p.cells += (int64_t)(m + 1) * ((int64_t)go[t1 - 1] - go[t0 - 1] + (t1 - t0));
   }
   *out = p;
 }
@@ -245,7 +280,9 @@ void plan_range(const saru_batch *b, int lo, int hi, PlanPart *out) {
 // ranges; the parts merged in order (bad: the first invalid candidate).
 PlanPart plan_span(const saru_batch *b, int lo, int hi) {
   const long n = hi - lo;
-  int nt = (int)std::min<long>(16, std::max<long>(1, n / 65536));
+  // (262k candidates take one thread 0.2 ms; a thread can take longer to start,
+  // right after large allocations several ms)
+  int nt = (int)std::min<long>(16, std::max<long>(1, n / 262144));
   const int hw = (int)std::thread::hardware_concurrency();
   if (hw > 0 && nt > hw) nt = hw;
   std::vector<PlanPart> parts((size_t)nt);
@@ -653,21 +690,38 @@ int run_full(Lane &L, const saru_batch *hb, const saru_batch *db, const saru_res
 // slice is a launch over candidates [t0, t1) of the whole call on the
 // device, so its tiles, and every output byte, are the ones the unsplit
 // launch makes; only candidate 0 of the call takes the first-of-call rule.
-// With pinned host buffers the copies run asynchronously; with pageable
-// ones they are correct but serialised.
 //
-// A slice holds up to kSliceBytes of inputs and slots, so that the first
-// kernel starts and the first results leave early: a power of two of
-// candidates, at most kSplitMost; a call of more than kSplitParts such slices
-// has kSplitParts larger ones (each costs nine calls into the driver).  176k
-// candidates of 100 bp (79 MB): 1.85 ms whole, 1.78 / 1.54 / 1.34 / 1.37 in
-// slices of 4 / 8 / 16 / 32 MB; 1.2M: 11.3 ms whole, 8.3 in slices of 16 MB.
+// With page-locked host arrays the copies run asynchronously, and a slice
+// holds up to kSliceBytes of inputs and slots, so that the first kernel starts
+// and the first results leave early: a power of two of candidates, at most
+// kSplitMost; a call of more than kSplitParts such slices has kSplitParts larger
+// ones (each costs nine calls into the driver).  176k candidates of 100 bp
+// (79 MB): 1.85 ms whole, 1.78 / 1.54 / 1.34 / 1.37 in slices of 4 / 8 / 16 /
+// 32 MB; 1.2M: 11.3 ms whole, 8.3 in slices of 16 MB.  Copies of pageable arrays
+// are serialised through the driver's own buffers, and a slice more only
+// costs (176k: 4.4-5.3 ms whole, 5.7-8.1 in slices of 16 MB), so such a call
+// is split from two slices of kSplitMost candidates on.
 constexpr long kSliceBytes = 16L << 20;
 constexpr long kSplitMost = 1L << 18;
 constexpr long kSplitParts = 32;
+// A call of fewer candidates is checked whole before its first launch, so that
+// a refused call leaves the caller's results as they were, while the copies in
+// of its first kAhead slices stream; a larger one slice by slice.
+constexpr long kCheckFirst = 2 * kSplitMost;
+constexpr long kAhead = 3;
 
-long split_chunk(const saru_batch *b) {
+bool page_locked(const void *p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeHost;
+}
+
+long split_chunk(const saru_batch *b, bool locked) {
   const long n = b->n;
+  if (!locked) return std::max(kSplitMost, ((n + kSplitParts - 1) / kSplitParts + 31) & ~31L);
   const double bytes = 2.0 * (double)b->genome_bytes + 2.0 * (double)b->total_slots;
   // (sizes that make no sense are refused later)
   const double fit = bytes > 0 ? (double)kSliceBytes / bytes * (double)n : (double)kSplitMost;
@@ -705,19 +759,18 @@ int check_slice_edges(const saru_batch *b, long chunk) {
   return SARU_OK;
 }
 
-// Copies in, slice by slice, on the lane's first stream.
-int upload_slices(Lane &L, const saru_batch *b, long chunk) {
+// Copies in of slices i0 .. i1 - 1, on the lane's first stream.
+int upload_slices(Lane &L, const saru_batch *b, long chunk, long i0, long i1) {
   const long n = b->n;
-  const size_t nslices = (size_t)((n + chunk - 1) / chunk);
-  while (L.ev_in.size() < nslices) {
+  while ((long)L.ev_in.size() < i1) {
     cudaEvent_t e;
     SARU_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     L.ev_in.push_back(e);
   }
   cudaStream_t si = L.stream;
   const int32_t *go = b->genome_offsets, *ro = b->read_offsets;
-  for (long t0 = 0, i = 0; t0 < n; t0 += chunk, ++i) {
-    const long t1 = std::min(n, t0 + chunk);
+  for (long i = i0; i < i1; ++i) {
+    const long t0 = i * chunk, t1 = std::min(n, t0 + chunk);
     const long g0 = t0 ? go[t0 - 1] : 0, g1 = go[t1 - 1];
     const long r0 = t0 ? ro[t0 - 1] : 0, r1 = ro[t1 - 1];
     SARU_CUDA(cudaMemcpyAsync(L.genome.as<char>() + g0, b->genome + g0, (size_t)(g1 - g0),
@@ -735,13 +788,16 @@ int upload_slices(Lane &L, const saru_batch *b, long chunk) {
   return SARU_OK;
 }
 
-// Kernels and copies out of the slices (after upload_slices), each slice
-// checked on the host (plan_range, threaded) just before its launch, so the
-// first kernels and copies out start while later slices are checked.  The
-// banded path was chosen from facts known up front (unit costs, k <= 15, the
-// first read's length); a slice whose reads differ in length or whose
-// windows are not m + so + eo sets *exact and launches stop (the call then
-// takes the exact path whole); an invalid candidate anywhere is an error.
+// Kernels and copies out of the slices (after upload_slices).  checked: the
+// plan of the whole call (banded), whose slices from kAhead on are copied in
+// here, as many ahead.  Without one each slice is checked on the
+// host (plan_range, threaded) just before its launch, so the first kernels and
+// copies out start while later slices are checked.  The banded path was then
+// chosen from facts known up front (unit costs, k <= 15, the first read's
+// length); a slice whose reads differ in length or whose windows are not
+// m + so + eo sets *exact and launches stop (the call then takes the exact path
+// whole); an invalid candidate anywhere is an error.
+
 // Host outputs of a call in compact records (saru_align_host_compact).
 struct HostCompact {
   int32_t *scores;
@@ -749,7 +805,7 @@ struct HostCompact {
   long rec_bytes;
 };
 
-int band_slices(Lane &L, const saru_batch *b, int m0, const saru_batch &db,
+int band_slices(Lane &L, const saru_batch *b, int m0, const Plan *checked, const saru_batch &db,
                 const saru_result &dr, const saru_result *r, int dev, long chunk, bool *exact,
                 const HostCompact *hc) {
   const long n = b->n, k = b->k;
@@ -766,14 +822,20 @@ int band_slices(Lane &L, const saru_batch *b, int m0, const saru_batch &db,
   int bad = -1;
   for (long t0 = 0, i = 0; t0 < n; t0 += chunk, ++i) {
     const long t1 = std::min(n, t0 + chunk);
-    const PlanPart part = plan_span(b, (int)t0, (int)t1);
-    if (part.bad >= 0) {
-      bad = part.bad;
-      break;
+    if (checked) {
+      pl = *checked;
+      const long next = i + kAhead;
+      if (next * chunk < n && (rc = upload_slices(L, b, chunk, next, next + 1))) return rc;
+    } else {
+      const PlanPart part = plan_span(b, (int)t0, (int)t1);
+      if (part.bad >= 0) {
+        bad = part.bad;
+        break;
+      }
+      if (!part.uniform || part.m_first != m0 || !part.regular) *exact = true;
+      if (*exact) continue;  // check the rest, launch no more
+      pl.wide = k > 7 && part.start_gap;
     }
-    if (!part.uniform || part.m_first != m0 || !part.regular) *exact = true;
-    if (*exact) continue;  // check the rest, launch no more
-    pl.wide = k > 7 && part.start_gap;
     const long g0 = t0 ? go[t0 - 1] : 0, g1 = go[t1 - 1];
     SARU_CUDA(cudaStreamWaitEvent(sr, L.ev_in[(size_t)i], 0));
     saru_batch slice = db;
@@ -810,15 +872,35 @@ int band_slices(Lane &L, const saru_batch *b, int m0, const saru_batch &db,
   return SARU_OK;
 }
 
+// The slice length of a host call that is split, 0 for one that is not.
+long host_chunk(const saru_batch *b, const saru_result *r, const HostCompact *hc) {
+  if (b->n <= 0 || b->k < 0) return 0;
+  long chunk = split_chunk(b, true);
+  if (b->n < 2 * chunk) return 0;
+  const int dev = current_device();
+  bool locked = dev >= 0 && cudaSetDevice(dev) == cudaSuccess;
+  for (const void *p : {(const void *)b->genome, (const void *)b->reads,
+                        (const void *)b->genome_offsets, (const void *)b->read_offsets,
+                        (const void *)b->dirs, hc ? (const void *)hc->scores : r->scores,
+                        hc ? (const void *)hc->records : r->read_aln,
+                        hc ? (const void *)hc->records : r->genome_aln})
+    locked = locked && page_locked(p);
+  if (!locked) chunk = split_chunk(b, false);
+  return b->n >= 2 * chunk ? chunk : 0;
+}
+
 // A host call: slot strings into r, or (hc) compact records.
 int align_host_impl(const saru_batch *b, saru_result *r, Lane &L, float *ms_out,
                     const HostCompact *hc = nullptr) {
   Plan pl;
   int rc;
-  const long chunk = b->n > 0 && b->k >= 0 ? split_chunk(b) : 0;
-  const bool big = chunk > 0 && b->n >= 2 * chunk;
+  const long chunk = host_chunk(b, r, hc);
+  const bool big = chunk > 0, checked = big && b->n < kCheckFirst;
   if (!big && (rc = plan_host(b, &pl))) return rc;
-  if (big && (rc = check_slice_edges(b, chunk))) return rc;
+  if (big && (rc = check_slice_edges(b, chunk))) {
+    const int whole = checked ? plan_host(b, &pl) : rc;  // names the candidate
+    return whole ? whole : rc;
+  }
   const int dev = current_device();
   if (dev < 0) {
     set_error("no CUDA device");
@@ -841,8 +923,26 @@ int align_host_impl(const saru_batch *b, saru_result *r, Lane &L, float *ms_out,
   const CompactOut dcmp{L.records.as<uint8_t>(), hc ? hc->rec_bytes : 0};
   SARU_CUDA(cudaMemsetAsync(L.status.p, 0, sizeof(int), s));
   bool split = false;
-  if (big) {  // copies in first; the host's checks run while they stream
-    if ((rc = upload_slices(L, b, chunk))) return rc;
+  const long nslices = big ? (b->n + chunk - 1) / chunk : 0;
+  if (checked) {  // the first copies in stream while the whole call is checked
+    const long ahead = std::min(nslices, kAhead);
+    if (!(rc = upload_slices(L, b, chunk, 0, ahead))) rc = plan_host(b, &pl);
+    if (!rc && !pl.band) rc = upload_slices(L, b, chunk, ahead, nslices);
+    if (!rc && pl.band && hc && hc->rec_bytes < saru::compact_record_bytes(pl.max_m, b->k)) {
+      set_error("record_bytes %ld < saru_compact_record_bytes(%d, %d)", hc->rec_bytes, pl.max_m,
+                b->k);
+      rc = SARU_E_INVALID;
+    }
+    if (rc) {
+      cudaStreamSynchronize(s);
+      return rc;
+    }
+    bool exact = false;
+    split = pl.band;
+    if (split && (rc = band_slices(L, b, pl.max_m, &pl, db, dr, r, dev, chunk, &exact, hc)))
+      return rc;
+  } else if (big) {  // copies in first; the host's checks run while they stream
+    if ((rc = upload_slices(L, b, chunk, 0, nslices))) return rc;
     const int m0 = b->read_offsets[0];
     split = b->match == 0 && b->mismatch == 1 && b->k <= 15 && m0 > 3 * b->k &&
             m0 <= saru::kMaxBandM && m0 >= 2;
@@ -852,7 +952,8 @@ int align_host_impl(const saru_batch *b, saru_result *r, Lane &L, float *ms_out,
       return SARU_E_INVALID;
     }
     bool exact = false;
-    if (split && (rc = band_slices(L, b, m0, db, dr, r, dev, chunk, &exact, hc))) return rc;
+    if (split && (rc = band_slices(L, b, m0, nullptr, db, dr, r, dev, chunk, &exact, hc)))
+      return rc;
     if (!split || exact) {
       split = false;
       if ((rc = plan_host(b, &pl))) {

@@ -311,10 +311,12 @@ SARU_HD bool position_hit(const FilterShape &S, int dr, const Lists &L, int a, u
   const int k = S.k, half = S.half, q = S.q;
   const int first = a == 0 ? 1 : 0;
   const int gs = (int)(pa - ((uint32_t)a * q + 1));
+  // a position in 32 bits without a sign: chunks may begin beyond 2^31
+  const int64_t at = (int64_t)(uint32_t)gs;
   int need = S.tresh - 1;  // hits up to the one that reaches the threshold
   if (need < 1) return false;
   for (int b = a + 1; b < half; ++b) {
-    const int64_t want = (int64_t)gs + (int64_t)b * q + 1;
+    const int64_t want = at + (int64_t)b * q + 1;
     need -= pair_hits(L, b, S.P, off, PosRange(want - k, want + k), need);
     if (need > 0) continue;
     if (first) {
@@ -331,7 +333,7 @@ SARU_HD bool position_hit(const FilterShape &S, int dr, const Lists &L, int a, u
     if (lim < 0) lim = -lim;
     const uint32_t ns = (uint32_t)(half - b - 1) * q + 1 + S.rest;
     if (L.len(half + b) == 0 || L.value(half + b, 0) == 0) continue;
-    const int64_t want = (int64_t)gs + (int64_t)ns;
+    const int64_t want = at + (int64_t)ns;
     need -= count_range(L, half + b, 0, PosRange(want - lim, want + lim), need);
     if (need > 0) continue;
     if (first) {

@@ -212,7 +212,7 @@ def measured_peaks() -> dict:
 
 
 def profile_traffic() -> dict | None:
-    """DRAM bytes per candidate of the banded kernel from the committed ncu
+    """DRAM bytes per candidate of the diagonal kernel from the committed ncu
     summary (profiles/diag_kernel_c2.json), if present."""
     p = ROOT / "profiles" / "diag_kernel_c2.json"
     if p.exists():

@@ -100,7 +100,7 @@ typedef struct {
 
 typedef struct {
   int32_t *scores;              /* n: D[L][m] when <= k; above k, k + 1 from the
-                                   banded kernel or the exact D[L][m] from the
+                                   diagonal kernel or the exact D[L][m] from the
                                    full-rectangle path (never printed either way) */
   char *read_aln;               /* total_slots bytes, reference slot layout */
   char *genome_aln;             /* total_slots bytes */
@@ -159,7 +159,7 @@ int saru_align_host_compact(const saru_batch *batch, int32_t *scores, uint8_t *r
 
 /* Device buffers in and out, enqueued on `stream` (a cudaStream_t, may be
  * NULL for the legacy stream).  Returns after enqueueing; completion is
- * ordered on the stream.  Runs the banded kernel only (unit costs, k <= 15,
+ * ordered on the stream.  Runs the diagonal kernel only (unit costs, k <= 15,
  * one read length m > 3k with m <= max_read_length <= 512); candidates it
  * cannot take are reported in result->status, with score k + 1.  `scratch`
  * must be 16-byte aligned and hold saru_scratch_bytes(n, max_read_length,
@@ -187,19 +187,19 @@ int saru_align_device(const saru_batch *batch, saru_result *result, void *scratc
 #define SARU_STATIC_SCRATCH_BYTES (32u << 20)
 int saru_align_device_static(const saru_batch *batch, saru_result *result, void *stream);
 
-/* Launch shape of the banded kernel for calls of one (read length, k):
+/* Launch shape of the alignment kernel for calls of one (read length, k):
  * the autotuner (saruman_b200.autotune) times the shapes on a sample and
- * installs the fastest here; every entry point that launches the banded
+ * installs the fastest here; every entry point that launches the
  * kernel for that class (saru_scratch_bytes included) then uses it.  0 in
- * a field keeps the default: as many warps per CTA (up to 4) and CTAs per
- * SM as fit.  word_bits sizes the scratch only (32-bit band words when
+ * a field keeps the default: the warps per CTA (up to 4) that keep the most
+ * warps on an SM, and as many CTAs per SM as fit.  word_bits sizes the scratch only (32-bit band words when
  * k <= 7 and 64-bit ones above by default).  A
  * multi-call launch looks up its class by (longest read, largest k).
  * Results do not depend on the shape.  Not in the reference. */
 typedef struct {
   int32_t warps_per_cta; /* 1..4: alignments per CTA = 32 x warps */
   int32_t ctas_per_sm;   /* cap on resident CTAs per SM */
-  int32_t word_bits;     /* 64: 64-bit band words for k <= 7 too; 32 only for k <= 7 */
+  int32_t word_bits;     /* sizes the scratch only; 32 only for k <= 7 */
 } saru_tuning;
 int saru_tuning_set(int32_t read_length, int32_t k, const saru_tuning *t); /* NULL: remove */
 int saru_tuning_get(int32_t read_length, int32_t k, saru_tuning *t);       /* 1 if set */
@@ -207,7 +207,7 @@ void saru_tuning_clear(void);
 
 /* ---- cost model of the autotuner (costmodel.cu) -----------------------------
  * A fully connected network, dims[0] inputs -> ... -> dims[nlayers] = 1
- * output, tanh hidden layers, fp32, that predicts the banded kernel's log
+ * output, tanh hidden layers, fp32, that predicts the alignment kernel's log
  * time per candidate from a bin's features and a launch shape; the
  * autotuner times only the shapes it ranks best.  Parameters: per layer
  * W (fan_out x fan_in, row-major) then the bias.  x: n rows of dims[0]
@@ -226,7 +226,7 @@ int saru_mlp_adam_step(float *params, const float *grad, float *m, float *v, int
                        float lr, float beta1, float beta2, float eps, int32_t step, void *stream);
 
 /* ---- compact results (no counterpart in the reference) ---------------------
- * The banded kernel can return, instead of the two slot strings of each
+ * The diagonal kernel can return, instead of the two slot strings of each
  * candidate (2(L + k) bytes), a fixed-size record of its traceback steps,
  * 2 bits each: record_bytes = saru_compact_record_bytes(m, k), 48 bytes for
  * m = 100, k = 5 against ~230 for the slots.  Word 0 of a record: the step
@@ -332,7 +332,7 @@ int32_t saru_genome_next(saru_genome_reader *g, char *out, int64_t *len, int64_t
                          int64_t *total);
 void saru_genome_close(saru_genome_reader *g);
 
-/* Device scratch the banded kernel needs for a batch (bytes). */
+/* Device scratch a batch must be given (bytes). */
 size_t saru_scratch_bytes(int32_t n, int32_t read_length, int32_t k, int wide);
 
 /* Several calls at once: each saru_batch is one reference-style call (its
@@ -369,7 +369,7 @@ int saru_align_multi_device_compact(const saru_batch *calls, saru_result *result
  * saru_align_multi_device request, while the next group's inputs are copied
  * in and the previous group's results are copied out.  Each request's
  * results are those saru_align_host gives for each of its calls: calls the
- * banded kernel flags (rare bytes, irregular windows, m <= 3k) are redone on
+ * diagonal kernel flags (rare bytes, irregular windows, m <= 3k) are redone on
  * the exact path before the request completes.
  * pipeline = 0 processes one request at a time, one launch per call and no
  * overlap: the plain per-request loop, for comparison.
@@ -409,7 +409,7 @@ saru_server *saru_server_create(const saru_server_config *cfg);
  * destroyed.  Refused (SARU_E_INVALID) while requests are unfinished. */
 int saru_server_set_genome(saru_server *s, const char *genome, int64_t genome_len);
 /* Queues a request; *ticket identifies it.  SARU_E_INVALID for calls the
- * banded kernel cannot take at all (costs, k, read length), SARU_E_NOMEM if
+ * diagonal kernel cannot take at all (costs, k, read length), SARU_E_NOMEM if
  * it can never fit the arena. */
 int saru_server_submit(saru_server *s, const saru_request *req, int64_t *ticket);
 /* Waits up to timeout_ms for a request: SARU_OK (results written),
@@ -498,7 +498,7 @@ uint64_t saru_kernel_launches(void);
 
 /* Diagnostics: 32-bit integer operations per second the current GPU
  * sustains on independent logic/add/shift chains at full occupancy (the
- * denominator of the banded kernel's roofline); -1 on error. */
+ * denominator of the alignment kernel's roofline); -1 on error. */
 double saru_int32_issue_probe(int iters);
 
 #ifdef __cplusplus

@@ -603,7 +603,7 @@ class Server:
 
 
 def set_tuning(m: int, k: int, warps: int = 0, ctas_per_sm: int = 0, word_bits: int = 0) -> None:
-    """Launch shape of the banded kernel for (read length, k) (saru_tuning_set)."""
+    """Launch shape of the alignment kernel for (read length, k) (saru_tuning_set)."""
     t = SaruTuning(warps, ctas_per_sm, word_bits)
     rc = load().saru_tuning_set(m, k, C.byref(t))
     if rc != SARU_OK:

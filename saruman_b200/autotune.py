@@ -1,7 +1,7 @@
-"""Autotuner of the banded kernel's launch shape per (read length, k).
+"""Autotuner of the alignment kernel's launch shape per (read length, k).
 
-A shape is (warps per CTA, CTAs per SM cap, band word bits); 0 keeps the
-library's default for that field.  For one (m, k) bin the tuner aligns a
+A shape is (warps per CTA, CTAs per SM cap, word bits, which size the scratch
+only); 0 keeps the library's default for that field.  For one (m, k) bin the tuner aligns a
 sample batch of that bin with every shape of the search space, timed with
 CUDA events on the device, and installs the fastest through
 saru_tuning_set.  Results are identical for every shape (the parity tests
@@ -89,7 +89,7 @@ class Sample:
 
 def time_shape(sample: Sample, shape: tuple[int, int, int], reps: int = 5,
                warmup: int = 2) -> float:
-    """Median milliseconds of one banded launch of the sample with `shape`."""
+    """Median milliseconds of one launch of the sample with `shape`."""
     import torch
     import saruman_b200 as S
     b = sample.batch

@@ -22,7 +22,7 @@ LIB = PKG / "libsaruman_b200.so"
 SOURCES = ["kernels.cu", "gather.cu", "filter.cu", "abi.cu", "writer.cpp", "server.cpp", "compact.cpp", "sam.cpp",
            "costmodel.cu", "probe.cu", "input.cpp"]
 HEADERS = ["kernels.cuh", "saru_core.cuh", "band_tile.cuh", "diag_tile.cuh", "writer.h", "server_internal.h",
-           "filter_core.cuh", "filter_calls.h"]
+           "filter_core.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler",
               "-fPIC,-O3,-Wall", "-Xptxas", "-v"]

@@ -1,6 +1,6 @@
 """Learned cost model of the autotuner.
 
-A small tanh network predicts the banded kernel's log time per candidate
+A small tanh network predicts the alignment kernel's log time per candidate
 for a (read length, k, start-gap fraction, candidates) bin and a launch
 shape.  It is trained on the GPU by the library's own kernels
 (saru_mlp_loss_grad, saru_mlp_adam_step: forward, backward and Adam in

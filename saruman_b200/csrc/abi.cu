@@ -4,7 +4,7 @@
 // Flow of one call (reference: src/cuda-functions.cu:586-1049):
 //   validate the call layout on the host and pick the kernel path
 //   H2D of windows, reads, offsets and flags on the caller's lane stream
-//   banded kernel (or the exact full-rectangle kernels) writes scores and
+//   diagonal kernel (or the exact full-rectangle kernels) writes scores and
 //     the two alignment-slot arrays, zero-filled, in the reference layout
 //   D2H of scores and slots; the TSV writer runs on the host
 // Each lane (forward / reverse caller) owns a stream and grow-only device
@@ -195,13 +195,13 @@ int sm_count(int dev) {
 // ---------------------------------------------------------------------------
 
 struct Plan {
-  bool band = false;   // banded kernel
-  bool wide = false;   // 64-bit band
+  bool band = false;   // diagonal kernel (errors within a band of k)
+  bool wide = false;   // scratch sized for 64-bit band words
   int max_m = 0;
   int64_t total_cells = 0;  // full-rectangle arena cells
 };
 
-// Host-side check of a host batch: the banded kernel needs unit costs, one
+// Host-side check of a host batch: the diagonal kernel needs unit costs, one
 // read length m > 3k with m <= kMaxBandM, k <= 15, and windows of exactly
 // m + so + eo bytes (the layout src/hash.c:986-1059 builds).
 // One range of candidates of plan_host's pass.
@@ -360,7 +360,6 @@ int smem_per_sm(int dev) {
   return v > 0 ? v : 228 * 1024;
 }
 
-// persistent grid of the banded kernel: as many CTAs as fit on the GPU
 // Launch shapes chosen per (read length, k) by the autotuner (saru_tuning_set);
 // classes without an entry keep the default shape.
 std::mutex g_tune_mu;
@@ -385,9 +384,9 @@ size_t band_scratch_bytes(long grid, int max_m, int k, bool wide) {
   return saru::band_scratch_bytes(grid, max_m, k, wide || tn.word_bits == 64, tn.warps);
 }
 
-// Enqueues the banded kernel on device buffers: calls[0..ncalls) as the
+// Enqueues the diagonal kernel on device buffers: calls[0..ncalls) as the
 // segments of one launch (the single-call entry points pass one).  Scratch:
-// the tile counter, then the decision planes of the persistent grid.
+// the tile counter (its stated size is an earlier form's, kernels.cu).
 using saru::CompactOut;
 
 // t0 > 0 (a multiple of 32, one call): align candidates t0 .. n - 1 only.
@@ -560,7 +559,7 @@ int run_band_classes(const saru_batch *calls, const saru_result *res, int ncalls
     return SARU_E_INVALID;
   }
   auto launch = [&](const LaunchClass &L, cudaStream_t st) {
-    Plan pl;  // a class of k > 7 calls runs 64-bit band words, even with one call
+    Plan pl;  // (a class of k > 7 calls has the larger scratch, even with one call)
     pl.band = true;
     pl.wide = L.wide;
     std::vector<saru_batch> cb;
@@ -1237,7 +1236,7 @@ int saru_align_device(const saru_batch *batch, saru_result *result, void *scratc
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// Entry point without any device allocation.  Its scratch (the banded
+// Entry point without any device allocation.  Its scratch (the
 // kernel's tile counter) is at the start of this file-scope device array,
 // present on every GPU that loads the library for the life of the process.
 // ---------------------------------------------------------------------------

@@ -1,6 +1,6 @@
 // compact.cpp -- host expansion of compact result records into the
 // reference's slot strings (the layout src/cuda-functions.cu:807-824 copies
-// back), byte for byte what the banded kernel writes in slot mode.
+// back), byte for byte what the diagonal kernel writes in slot mode.
 #include <stdint.h>
 #include <string.h>
 

@@ -1,6 +1,6 @@
 // costmodel.cu -- forward, backward and Adam kernels of the autotuner's
 // cost model: a small fully connected network (tanh hidden layers, linear
-// output) that predicts the banded kernel's log time per candidate from a
+// output) that predicts the alignment kernel's log time per candidate from a
 // bin's features and a launch shape.  fp32 throughout; every reduction runs
 // in a fixed order (one thread per output, a sequential loop over the
 // samples), so gradients are deterministic and comparable with a CPU

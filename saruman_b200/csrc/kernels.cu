@@ -300,8 +300,8 @@ __device__ __forceinline__ int diag_tile(const KernelArgs &a, const TileAhead &n
   return st;
 }
 
-// 16 warps an SM: registers (106 a thread) and slices (13.8 KB at 100 bp, k = 5)
-// both end there.  Held to 3 or 5 CTAs of 4 warps: 332 or
+// 16 warps an SM: registers (106 a thread in the rows form, 128 in the planes
+// forms) and slices (13.8 KB at 100 bp, k = 5) both end there.  Held to 3 or 5 CTAs of 4 warps: 332 or
 // 294 us against 291 for 930k candidates of 100 bp.
 constexpr int kDiagCtas = 4;
 constexpr int kDiagWarpsPerSm = 4 * kDiagCtas;
@@ -607,8 +607,8 @@ cudaError_t allow_smem() {
 }
 }  // namespace
 
-// The largest slice a launch's segments need (a slice does not grow with
-// the read length and k in every case, so it is not the longest read's).
+// The largest slice a launch's segments need (the longest reads and the
+// largest k may be different segments').
 long diag_slice(const KernelArgs &a, bool rows) {
   const int cell = a.max_m <= kByteColumns ? 1 : 2;
   long most = 0;

@@ -13,7 +13,7 @@ constexpr int kStatusOverflow = 4;   // a traceback left its slot / band
 constexpr int kStatusUndefined = 8;  // the reference would read outside its arrays
 constexpr int kStatusGather = 16;    // a gathered candidate lies outside the genome or read table
 
-constexpr int kMaxBandM = 512;  // longest read of the banded kernel
+constexpr int kMaxBandM = 512;  // longest read of the diagonal kernel
 constexpr int kMaxOpWords = (kMaxBandM + 3 * 15 + 15) / 16 + 1;
 
 // One reference-style call inside a launch: its own read length, k, band
@@ -51,7 +51,8 @@ struct KernelArgs {
 };
 
 // Launch shape of the alignment kernel for one (read length, k) class; 0
-// keeps the default (as many warps per CTA and CTAs per SM as fit).
+// keeps the default (the warps per CTA that keep the most warps on an SM, as
+// many CTAs as fit).
 struct Tuning {
   int warps = 0;        // warps per CTA, 1..4
   int ctas_per_sm = 0;  // cap on resident CTAs per SM

@@ -1,6 +1,6 @@
 // probe.cu -- measured integer-issue peak of the current GPU.
 //
-// The roofline of the banded kernel is integer issue (LOP3 / IADD / SHF
+// The roofline of the alignment kernel is integer issue (LOP3 / IADD / SHF
 // work, no tensor-core contraction).  This probe runs eight independent
 // chains of (lop3, add, funnel-shift) per thread at full occupancy and
 // reports 32-bit integer operations per second, the denominator the

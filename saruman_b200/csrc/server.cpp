@@ -4,7 +4,7 @@
 // out), typically one per read-length bin.  The scheduler thread admits
 // requests in arrival order while the device arena has room for their
 // inputs and outputs; the requests admitted together form a launch group
-// whose calls all go to one multi-call request of the banded kernel (one
+// whose calls all go to one multi-call request of the diagonal kernel (one
 // persistent launch per read-length class, classes concurrent).  Three
 // streams overlap the work: the inputs of group i+1 are copied in while
 // group i computes, and the completion thread copies group i's results out
